@@ -37,9 +37,21 @@ template <typename C>
 __device__ __forceinline__ C csub(C a, C b) {
   return mk(a.x - b.x, a.y - b.y);
 }
+// Products whose rounding is spelled out (one rounded product, one fused
+// multiply-add per part), so that every kernel that inlines the same body
+// gives the same bits whatever the compiler would contract there.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 template <typename C>
 __device__ __forceinline__ C cmul(C a, C b) {
-  return mk(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return mk(fma_rn(a.x, b.x, -mul_rn(a.y, b.y)), fma_rn(a.x, b.y, mul_rn(a.y, b.x)));
+}
+// i (ka a - kb b): one component of the curl i k x v.
+template <typename C, typename T>
+__device__ __forceinline__ C curl_part(T ka, C a, T kb, C b) {
+  return mk(fma_rn(kb, b.y, -mul_rn(ka, a.y)), fma_rn(ka, a.x, -mul_rn(kb, b.x)));
 }
 // (0, k) * z, the product std::complex forms for i*k*z.
 template <typename C, typename T>

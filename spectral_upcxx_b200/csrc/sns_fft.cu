@@ -72,9 +72,10 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_trigger();
   pdl_wait();
-  line_pass_tile<T, L, PRO, ParamFields, ORD>(geo, ParamFields{f}, f.n, tw, sg, scale, flags,
-                                               wshift, (int64_t)blockIdx.x,
-                                               reinterpret_cast<cx_t<T>*>(smem_raw));
+  line_pass_tile<T, L, PRO, ParamFields, ORD>(
+      geo, ParamFields{f}, f.n, tw, sg, scale, flags, wshift,
+      tile_order((int64_t)blockIdx.x, (int64_t)gridDim.x, geo.rev),
+      reinterpret_cast<cx_t<T>*>(smem_raw));
 }
 
 // epilogue-only pass (used when every axis has length 1)
@@ -129,6 +130,7 @@ static int launch_pass(const LineGeo& geo, const FieldPtrs& f, int sign, int fla
   }
   LineGeo g = geo;
   g.pf = tiles_in_waves(k_line_pass<T, L, PRO, ORD>, threads, smem, geo.pfw);
+  if (g.rev) g.pf = -g.pf;
   cudaError_t e = launch_pdl(k_line_pass<T, L, PRO, ORD>, dim3((unsigned)blocks), dim3(threads),
                              smem, stream, g, f, tw, (T)sign, (T)scale, flags, wshift);
   if (e != cudaSuccess) return cuda_status(e, "k_line_pass");
@@ -317,9 +319,17 @@ int fft3d(void* const* fields, int nf, int nx, int ny, int nz, int sign, int fla
       tuned = fft3d_tuned(nx, ny, nz, nf, prec, &tc);
     }
   }
+  // The y pass of a forward transform and the z and x passes of an inverse one
+  // walk their tiles from the last to the first: x and y tiles both follow the
+  // z planes, and an inverse often follows a forward transform's z pass, so
+  // each starts on what the pass before it left in L2 (256^3 complex64 forward +
+  // inverse on B200: 0.293 ms against 0.303 in plain order).
   auto geo = [&](int axis) {
-    return tuned ? axis_geo(axis, nx, ny, nz, prec, tc.wmax[axis], tc.tmax[axis], tc.ord[axis])
-                 : axis_geo(axis, nx, ny, nz, prec);
+    LineGeo g = tuned ? axis_geo(axis, nx, ny, nz, prec, tc.wmax[axis], tc.tmax[axis],
+                                 tc.ord[axis])
+                      : axis_geo(axis, nx, ny, nz, prec);
+    g.rev = (sign < 0) == (axis == 1);
+    return g;
   };
   // a pass of the plan: the TMA-staged form where the tuned plan chose it
   // (SNS_FFT_TMA = 1 or 2 stages asks for it on the passes of an untuned

@@ -82,8 +82,11 @@ struct LineGeo {
   int kx_half;
   // radix order of the line FFT (RadixOrder; plain-load passes of 64..1024)
   int ord;
+  // walk the tiles from the last to the first (tile_order)
+  int rev;
   // L2 prefetch: each CTA asks L2 for the inputs of the tile pf launches
-  // ahead (0: none); the launcher sets pf to pfw waves of resident CTAs
+  // ahead in the walk (0: none; negative in a reversed walk); the launcher
+  // sets it to pfw waves of resident CTAs
   int64_t pf;
   int pfw;
 };

@@ -136,7 +136,7 @@ __device__ __forceinline__ void dft(C* a, T sg) {
       } else {
         constexpr int step = 16 / R;
         const T c = (T)tw16_c(k * step), s = sg * (T)tw16_s(k * step);
-        t = mk(o[k].x * c - o[k].y * s, o[k].x * s + o[k].y * c);
+        t = cmul(o[k], mk(c, s));
       }
       a[k] = cadd(e[k], t);
       a[k + H] = csub(e[k], t);

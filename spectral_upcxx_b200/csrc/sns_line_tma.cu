@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
   __syncthreads();
   // the fields are written by the pass before
   pdl_wait();
-  auto issue = [&](int64_t blk, int k) {  // thread 0
+  auto issue = [&](int64_t b, int k) {  // thread 0
+    const int64_t blk = tile_order(b, ntiles, geo.rev);
     const int fld = (int)(blk % nf);
     const int64_t t = blk / nf;
     const CUtensorMap* m = pick_map(fld, m0, m1, m2, m3, m4, m5);
@@ -139,7 +140,8 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
       return;
     }
     line_pass_tile_staged<T, L, ParamFields, ORD>(geo, ParamFields{f}, nf, tw, sg, scale, flags,
-                                                  wshift, blk, stage0 + k * per, rows, [&] {
+                                                  wshift, tile_order(blk, ntiles, geo.rev),
+                                                  stage0 + k * per, rows, [&] {
                                                     if (S == 1) {
                                                       __syncthreads();
                                                       if (threadIdx.x == 0 && more) {

@@ -36,11 +36,12 @@ namespace sns {
 // K3: x lines -- inverse 6 fields, cross product, forward 3 fields.
 template <typename T, int L>
 __global__ void __launch_bounds__(MaxThreads<T>::value)
-    k_xcross(FieldPtrs f, const cx_t<T>* __restrict__ tw, int G, T scale2, int64_t pf) {
+    k_xcross(FieldPtrs f, const cx_t<T>* __restrict__ tw, int G, T scale2, int64_t pf, int rev) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_trigger();
   pdl_wait();
-  xcross_tile<T, L>(ParamFields{f}, tw, G, scale2, (int64_t)blockIdx.x, (int)blockDim.x,
+  xcross_tile<T, L>(ParamFields{f}, tw, G, scale2,
+                    tile_order((int64_t)blockIdx.x, (int64_t)gridDim.x, rev), (int)blockDim.x,
                     reinterpret_cast<cx_t<T>*>(smem_raw), pf, (int64_t)gridDim.x);
 }
 
@@ -49,11 +50,12 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 // latency, at the price of a few spilled registers.
 template <typename T, int L>
 __global__ void __launch_bounds__(192, 5)
-    k_xcross_occ(FieldPtrs f, const cx_t<T>* __restrict__ tw, int G, T scale2, int64_t pf) {
+    k_xcross_occ(FieldPtrs f, const cx_t<T>* __restrict__ tw, int G, T scale2, int64_t pf, int rev) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_trigger();
   pdl_wait();
-  xcross_tile<T, L>(ParamFields{f}, tw, G, scale2, (int64_t)blockIdx.x, (int)blockDim.x,
+  xcross_tile<T, L>(ParamFields{f}, tw, G, scale2,
+                    tile_order((int64_t)blockIdx.x, (int64_t)gridDim.x, rev), (int)blockDim.x,
                     reinterpret_cast<cx_t<T>*>(smem_raw), pf, (int64_t)gridDim.x);
 }
 
@@ -66,7 +68,7 @@ __global__ void __launch_bounds__(192, 5)
 template <typename T, int L>
 __global__ void __launch_bounds__(MaxThreads<T>::value)
     k_xcross_tma(FieldPtrs f, const cx_t<T>* __restrict__ tw, int G, T scale2, int64_t ntiles,
-                 int* err, long long stall_cycles) {
+                 int rev, int* err, long long stall_cycles) {
   using C = cx_t<T>;
   constexpr int E = LinePlan<L>::E, TPL = LinePlan<L>::TPL;
   constexpr int RS = xrow_stride(L, (int)sizeof(C));
@@ -85,7 +87,7 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
   __syncthreads();
   pdl_wait();  // the rows are written by the y pass before
   auto issue = [&](int64_t blk) {  // thread 0
-    const int64_t e0 = blk * per;
+    const int64_t e0 = tile_order(blk, ntiles, rev) * per;
     if ((tc::smem_u32(stage) & 127u) || ((e0 * (int64_t)sizeof(C)) & 15)) {
       atomicExch(err, 2);
       tma::arrive(&full[0]);
@@ -112,7 +114,8 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
       __syncthreads();
       return;
     }
-    xcross_tile_from<T, L>(ParamFields{f}, tw, G, scale2, blk, (int)blockDim.x, rows,
+    xcross_tile_from<T, L>(ParamFields{f}, tw, G, scale2, tile_order(blk, ntiles, rev),
+                           (int)blockDim.x, rows,
                            [&](int fld, int gl, int j, C (&v)[E]) {
                              const C* src = stage + fld * per + gl * L + j;
 #pragma unroll
@@ -143,7 +146,7 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 template <typename T, int M>
 __global__ void __launch_bounds__(384, sizeof(T) == 4 ? 2 : 1)
     k_xcross_r2c(FieldPtrs f, const cx_t<T>* __restrict__ twN, const cx_t<T>* __restrict__ twM,
-                 int G, T scale2) {
+                 int G, T scale2, int rev) {
   using C = cx_t<T>;
   using P = LinePlan<M>;
   constexpr int E = P::E, TPL = P::TPL, RS = xrow_stride(M, (int)sizeof(C));
@@ -152,7 +155,7 @@ __global__ void __launch_bounds__(384, sizeof(T) == 4 ? 2 : 1)
   pdl_trigger();
   pdl_wait();
   C* sm = reinterpret_cast<C*>(smem_raw);
-  const int64_t row0 = (int64_t)blockIdx.x * G;
+  const int64_t row0 = tile_order((int64_t)blockIdx.x, (int64_t)gridDim.x, rev) * G;
   const int per = G * M;
   const int j = threadIdx.x % TPL, line = threadIdx.x / TPL;
   const int fld = line / G, gl = line - fld * G;
@@ -250,11 +253,12 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_trigger();
   pdl_wait();
+  const int64_t blk = tile_order((int64_t)blockIdx.x, (int64_t)gridDim.x, geo.rev);
   if constexpr (RELOAD)
-    curl_zpass_tile_reload<T, L>(geo, ParamFields{f}, tw, wshift, (int64_t)blockIdx.x,
+    curl_zpass_tile_reload<T, L>(geo, ParamFields{f}, tw, wshift, blk,
                                  reinterpret_cast<cx_t<T>*>(smem_raw));
   else
-    curl_zpass_tile<T, L>(geo, ParamFields{f}, tw, wshift, (int64_t)blockIdx.x,
+    curl_zpass_tile<T, L>(geo, ParamFields{f}, tw, wshift, blk,
                           reinterpret_cast<cx_t<T>*>(smem_raw));
 }
 
@@ -299,7 +303,8 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
   __syncthreads();
   // V is written by the step before (its update pass)
   pdl_wait();
-  auto issue = [&](int64_t blk, int k) {  // thread 0
+  auto issue = [&](int64_t b, int k) {  // thread 0
+    const int64_t blk = tile_order(b, ntiles, geo.rev);
     const int u = (int)(sizeof(C) / 8);
     const int x0 = (int)((blk % geo.TA) * geo.W) * u, y0 = (int)((blk / geo.TA) * geo.G);
     C* st = stage0 + k * 3 * comp;
@@ -345,7 +350,8 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
       __syncthreads();
       return;
     }
-    curl_zpass_tile_staged<T, L>(geo, ParamFields{f}, tw, wshift, blk, stage0 + k * 3 * comp, rows,
+    curl_zpass_tile_staged<T, L>(geo, ParamFields{f}, tw, wshift,
+                                 tile_order(blk, ntiles, geo.rev), stage0 + k * 3 * comp, rows,
                                  [&] {
                                    if (S == 1) {
                                      __syncthreads();
@@ -525,7 +531,7 @@ int launch_xcross(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream
     const double N = (double)pl.nx * pl.ny * pl.nz;
     const int64_t pf = tiles_in_waves(k_xcross_occ<T, L>, threads, smem, pl.pf_waves);
     cudaError_t e = launch_pdl(k_xcross_occ<T, L>, dim3((unsigned)(rows / G)), dim3(threads), smem,
-                               s, f, tw, G, (T)(1.0 / (N * N)), pf);
+                               s, f, tw, G, (T)(1.0 / (N * N)), pl.rev ? -pf : pf, (int)pl.rev);
     if (e != cudaSuccess) return cuda_status(e, "k_xcross_occ");
     return OK;
   }
@@ -542,7 +548,7 @@ int launch_xcross(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream
   const int blocks = (int)(rows / G);
   const int64_t pf = tiles_in_waves(k_xcross<T, L>, threads, smem, pl.pf_waves);
   cudaError_t e = launch_pdl(k_xcross<T, L>, dim3(blocks), dim3(threads), smem, s, f, tw, G,
-                             (T)(1.0 / (N * N)), pf);
+                             (T)(1.0 / (N * N)), pl.rev ? -pf : pf, (int)pl.rev);
   if (e != cudaSuccess) return cuda_status(e, "k_xcross");
   return OK;
 }
@@ -606,7 +612,7 @@ int launch_xcross_tma(const NSPlan& pl, const FieldPtrs& f, int64_t rows, int* e
   }
   const double N = (double)pl.nx * pl.ny * pl.nz;
   e = launch_pdl(k_xcross_tma<T, L>, dim3((unsigned)blocks), dim3(threads), smem, s, f, tw, G,
-                 (T)(1.0 / (N * N)), ntiles, err, tma_stall_cycles());
+                 (T)(1.0 / (N * N)), ntiles, (int)pl.rev, err, tma_stall_cycles());
   if (e != cudaSuccess) return cuda_status(e, "k_xcross_tma");
   return OK;
 }
@@ -624,6 +630,7 @@ int launch_zcurl_as(const NSPlan& pl, const FieldPtrs& f, cudaStream_t s) {
   g.ny = pl.ny;
   g.nz = pl.nz;
   g.kx_half = pl.real;
+  g.rev = pl.rev;
   g.ps = (int64_t)pl.nx * pl.ny;
   g.gs = pl.nx;
   g.TA = pl.nx / g.W;
@@ -649,6 +656,7 @@ int launch_zcurl_as(const NSPlan& pl, const FieldPtrs& f, cudaStream_t s) {
   int wshift = 0;
   while ((1 << wshift) < g.W) wshift++;
   g.pf = tiles_in_waves(k_zcurl<T, L, RELOAD>, threads, smem, pl.pf_waves);
+  if (g.rev) g.pf = -g.pf;
   cudaError_t e = launch_pdl(k_zcurl<T, L, RELOAD>, dim3((unsigned)(g.TA * g.TB)), dim3(threads),
                              smem, s, g, f, tw, wshift);
   if (e != cudaSuccess) return cuda_status(e, "k_zcurl");
@@ -689,6 +697,7 @@ int launch_zcurl_tma(const NSPlan& pl, const FieldPtrs& f, int* err, cudaStream_
   g.ny = pl.ny;
   g.nz = pl.nz;
   g.kx_half = pl.real;
+  g.rev = pl.rev;
   g.ps = (int64_t)pl.nx * pl.ny;
   g.gs = pl.nx;
   g.TA = pl.nx / g.W;
@@ -767,7 +776,7 @@ int launch_xcross_r2c(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaSt
   }
   const double N = (double)pl.nx_phys * pl.ny * pl.nz;
   cudaError_t e = launch_pdl(k_xcross_r2c<T, M>, dim3((unsigned)(rows / G)), dim3(threads), smem,
-                             s, f, twN, twM, G, (T)(1.0 / (N * N)));
+                             s, f, twN, twM, G, (T)(1.0 / (N * N)), (int)pl.rev);
   if (e != cudaSuccess) return cuda_status(e, "k_xcross_r2c");
   return OK;
 }
@@ -1010,6 +1019,8 @@ int xpass(const NSPlan& pl, const FieldPtrs& f, int64_t rows, int* err, cudaStre
 
 int elems(int L) { return L >= 16 ? 16 : L; }
 
+constexpr double kL2Bytes = 126e6;  // L2 of the B200
+
 }  // namespace
 
 int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, bool real) {
@@ -1034,11 +1045,17 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
       return ERR_UNSUPPORTED;
     }
   const size_t esz = prec == PREC_C128 ? 16 : 8;
-  // K3 tile: G rows of all six fields
+  // fields beyond L2: the step streams from HBM
+  const bool big = 12.0 * esz * nx * ny * nz > kL2Bytes;
+  // K3 tile: G rows of all six fields, in CTAs of at most 192 threads
+  // (complex64) or 96 (complex128): small CTAs drift apart, so one CTA's loads
+  // run under another's transforms.  B200, 256^3: complex64 0.266 ms with 192
+  // threads, 0.283 with 96 and with 384; complex128 0.598 with 96, 0.614 with
+  // 192, 0.737 with 384.
   {
     const int TPL = nx / elems(nx);
     int G = 1;
-    while (6 * (G * 2) * TPL <= 384 && ((int64_t)ny * nz) % (G * 2) == 0 &&
+    while (6 * (G * 2) * TPL <= (prec == PREC_C128 ? 96 : 192) && ((int64_t)ny * nz) % (G * 2) == 0 &&
            (size_t)6 * G * 2 * xrow_stride(nx, (int)esz) * esz <= 110 * 1024)
       G *= 2;
     if (6 * G * TPL > max_threads(prec)) {
@@ -1147,10 +1164,11 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
           pl.update_blocks = (nx / w) * ny;
         }
     // L2 prefetch of each tile's V and C0 once its cross product's loads are
-    // in flight (SNS_Z_PFSELF=1; asked before those loads it delayed them and
-    // measured slower)
+    // in flight (asked before those loads it delayed them), where they come
+    // from HBM (SNS_Z_PFSELF = 0, 1).  B200, 256^3: complex64 0.389 ms against
+    // 0.469 without, complex128 0.776 against 0.894.
     const char* epf = getenv("SNS_Z_PFSELF");
-    pl.z_pfself = epf && epf[0] == '1';
+    pl.z_pfself = epf ? epf[0] == '1' : big;
     // closure update: nine fields in the tile
     const int cap = std::min(576, max_threads(prec));
     int Ws = 1;
@@ -1166,6 +1184,10 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   // thread-block-cluster pass over each plane (sns_xyc.cu; nx = ny = 128, or
   // 256 in complex64; 1.28 vs 0.73 ms at 256^3), SNS_XY_PASSES=1 the
   // persistent dataflow launch through L2 (sns_xy.cu; 1.09 vs 0.79 ms).
+  // K1 walks its tiles back from where K5 ended (both follow the xy plane),
+  // K3 back from where K2 ended (both follow z).  B200, whole complex64 step:
+  // 0.5 to 1 % at 256^3, 3.5 % at 128^3.
+  pl.rev = true;
   const char* env = getenv("SNS_XY_PASSES");
   const bool dataflow = env && env[0] == '1';
   pl.use_xy = !real && dataflow && xy_supported(nx, ny, prec) &&
@@ -1179,12 +1201,18 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   pl.lineW = lineW > 0 ? lineW : 0;
   pl.lineT = 0;
   pl.lineOrd = 0;
+  // y passes of fields beyond L2: one line group per CTA of up to 128 threads
+  // (or one run of W lines), in complex64 over TMA-staged tiles.  B200, 256^3,
+  // both passes: complex64 0.427 ms against 0.491 (direct loads, 256 threads);
+  // complex128 0.820 against 0.908 (256 threads; staged 0.87).
+  if (big && lineW <= 0 && !getenv("SNS_LINE_W")) pl.lineT = 128;
   {
-    // the y passes over TMA-staged tiles on request (SNS_Y_TMA = 1 or 2 stages)
+    // SNS_Y_TMA = 0 (direct loads), 1 or 2 stages
     const char* e = getenv("SNS_Y_TMA");
-    const int v = e ? atoi(e) : 0;
+    const int v = e ? atoi(e) : big && prec == PREC_C64 ? 1 : 0;
     pl.y_tma = 0;
-    if ((v == 1 || v == 2) && line_tma_ok(axis_geo(1, nx, ny, nz, prec), prec, v))
+    if ((v == 1 || v == 2) &&
+        line_tma_ok(axis_geo(1, nx, ny, nz, prec, pl.lineW, pl.lineT), prec, v))
       pl.y_tma = v;
   }
   pl.tuned = false;
@@ -1242,6 +1270,7 @@ int run_k1(const NSPlan& pl, void* const V[3], void* const U[6], int* err_word, 
                                 : zcurl<float>(pl, f, err_word, s);
   LineGeo g = axis_geo(2, pl.nx, pl.ny, pl.nz, pl.prec, pl.lineW);
   g.kx_half = pl.real;
+  g.rev = pl.rev;
   return run_line_pass(g, f, +1, 0, 1.0, pl.prec, s, PRO_CURL6);
 }
 

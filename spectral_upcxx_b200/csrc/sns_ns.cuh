@@ -27,6 +27,8 @@ struct NSPlan {
   bool k1_lines;      // K1 as a line pass of V and i kz V (5 fields into the work
                       // fields W), the curl formed in K2's prologue (PRO_OMEGA)
   int k1lW, k1lT;     // tile knobs of that z line pass (axis_geo wmax, tmax)
+  bool rev;           // K1 and K3 walk their tiles from the last to the first, so each
+                      // starts on what the pass before it left in L2
   int zW;             // adjacent z lines per CTA of the update pass
   int update_blocks;  // CTAs of the update pass (= diagnostics partials)
   int sgs_W;          // adjacent z lines per CTA of the closure update (9 fields)

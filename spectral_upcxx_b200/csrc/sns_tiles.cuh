@@ -48,6 +48,13 @@ __device__ __forceinline__ LineCoord line_coord(const LineGeo& geo, int64_t base
   return c;
 }
 
+// Tile of the b-th CTA of a pass over n tiles, walked from the last one when
+// rev: a pass that starts where the pass before it ended finds that pass's
+// last outputs (up to the size of L2) still there.
+__device__ __forceinline__ int64_t tile_order(int64_t b, int64_t n, int rev) {
+  return rev ? n - 1 - b : b;
+}
+
 // Ask L2 for the 128-byte line holding p (a hint: no register, no wait).
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
@@ -81,7 +88,7 @@ __device__ __forceinline__ void prefetch_lines(const char* src, int64_t base, in
 template <int L, typename C, typename Fields>
 __device__ __forceinline__ void prefetch_curl_tile(const LineGeo& geo, const Fields& f,
                                                    int64_t bp) {
-  if (geo.pf <= 0 || bp >= geo.TA * geo.TB) return;
+  if (geo.pf == 0 || bp < 0 || bp >= geo.TA * geo.TB) return;
   const int64_t basep = (bp % geo.TA) * geo.sa + (bp / geo.TA) * geo.sb;
 #pragma unroll
   for (int d = 0; d < 3; d++)
@@ -99,14 +106,14 @@ __device__ __forceinline__ C pro_load(const C* __restrict__ src, const C* __rest
                                       int field, int64_t idx, T kx, T ky, T kz) {
   if constexpr (PRO == PRO_CURL6) {
     if (field < 3) return src[idx];
-    if (field == 3) return csub(ikmul(ky, v2[idx]), ikmul(kz, v1[idx]));
-    if (field == 4) return csub(ikmul(kz, v0[idx]), ikmul(kx, v2[idx]));
-    return csub(ikmul(kx, v1[idx]), ikmul(ky, v0[idx]));
+    if (field == 3) return curl_part(ky, v2[idx], kz, v1[idx]);
+    if (field == 4) return curl_part(kz, v0[idx], kx, v2[idx]);
+    return curl_part(kx, v1[idx], ky, v0[idx]);
   } else if constexpr (PRO == PRO_OMEGA) {
     if (field < 3) return src[idx];
     if (field == 3) return csub(ikmul(ky, v2[idx]), d1[idx]);
     if (field == 4) return csub(d0[idx], ikmul(kx, v2[idx]));
-    return csub(ikmul(kx, v1[idx]), ikmul(ky, v0[idx]));
+    return curl_part(kx, v1[idx], ky, v0[idx]);
   } else {
     return src[idx];
   }
@@ -175,7 +182,7 @@ __device__ __forceinline__ void line_pass_tile(const LineGeo& geo, const Fields&
   if constexpr (PRO == PRO_LOAD || PRO == PRO_IKAXIS) {
     // with this tile's loads in flight, the tile pf launches ahead into L2
     const int64_t bp = blk + geo.pf;
-    if (geo.pf > 0 && bp < geo.TA * geo.TB * nf) {
+    if (geo.pf != 0 && bp >= 0 && bp < geo.TA * geo.TB * nf) {
       const int64_t tp = bp / nf;
       prefetch_lines<L>(reinterpret_cast<const char*>(f.in((int)(bp % nf))),
                         (tp % geo.TA) * geo.sa + (tp / geo.TA) * geo.sb, W, geo.G, geo.gs,
@@ -307,11 +314,11 @@ __device__ __forceinline__ void curl_zpass_tile(const LineGeo& geo, const Fields
       const T kz = (T)freq_i(j + TPL * e, geo.nz);
       C o;
       if (d == 0)
-        o = csub(ikmul(ky, r2[pp]), ikmul(kz, r1[pp]));
+        o = curl_part(ky, r2[pp], kz, r1[pp]);
       else if (d == 1)
-        o = csub(ikmul(kz, r0[pp]), ikmul(kx, r2[pp]));
+        o = curl_part(kz, r0[pp], kx, r2[pp]);
       else
-        o = csub(ikmul(kx, r1[pp]), ikmul(ky, r0[pp]));
+        o = curl_part(kx, r1[pp], ky, r0[pp]);
       rowW[pp] = o;
     }
   }
@@ -386,11 +393,11 @@ __device__ __forceinline__ void curl_zpass_tile_reload(const LineGeo& geo, const
       const T kz = (T)freq_i(j + TPL * e, geo.nz);
       const C a = pa[q], b = pb[q];
       if (d == 0)
-        v[e] = csub(ikmul(ky, a), ikmul(kz, b));
+        v[e] = curl_part(ky, a, kz, b);
       else if (d == 1)
-        v[e] = csub(ikmul(kz, a), ikmul(kx, b));
+        v[e] = curl_part(kz, a, kx, b);
       else
-        v[e] = csub(ikmul(kx, a), ikmul(ky, b));
+        v[e] = curl_part(kx, a, ky, b);
     }
   }
   // the last stage of the first transform read the row before a block barrier,
@@ -454,11 +461,11 @@ __device__ __forceinline__ void curl_zpass_tile_staged(const LineGeo& geo, const
       const T kz = (T)freq_i(j + TPL * e, geo.nz);
       const C a = pa[q], b = pb[q];
       if (d == 0)
-        v[e] = csub(ikmul(ky, a), ikmul(kz, b));
+        v[e] = curl_part(ky, a, kz, b);
       else if (d == 1)
-        v[e] = csub(ikmul(kz, a), ikmul(kx, b));
+        v[e] = curl_part(kz, a, kx, b);
       else
-        v[e] = csub(ikmul(kx, a), ikmul(ky, b));
+        v[e] = curl_part(kx, a, ky, b);
     }
   }
   after_reads();
@@ -552,7 +559,7 @@ __device__ __forceinline__ void xcross_tile(const Fields& f, const cx_t<T>* __re
     const int64_t i0 = (blk * G + gl) * L + j;
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = src[i0 + TPL * e];
-    if (pf > 0 && blk + pf < nblk) {
+    if (pf != 0 && blk + pf >= 0 && blk + pf < nblk) {
       // with this tile's loads in flight, the six input rows of tile blk + pf
       // into L2
 #pragma unroll
@@ -594,6 +601,40 @@ struct UpdateArgs {
   int pf_self;
 };
 
+// A divisor shared by several quotients.  FP64: the reciprocal once, each
+// quotient corrected by its remainder (as exact as a division, 3 operations
+// instead of a division's ten or so).  FP32: the reciprocal rounded once.
+template <typename T>
+struct Divisor {
+  T den, r;
+  __device__ __forceinline__ T under(T v) const {
+    if constexpr (sizeof(T) == 8) {
+      const T q = mul_rn(v, r);
+      const T e = fma_rn(-q, den, v);
+      return e == e ? fma_rn(e, r, q) : q;  // an infinite quotient stays infinite
+    } else {
+      return mul_rn(v, r);
+    }
+  }
+};
+// k2: a whole number below 2^24 (FP32).  The correctly rounded FP32 reciprocal
+// of an FP32 number is the FP64 one rounded once more (53 >= 2 x 24 + 2).
+__device__ __forceinline__ Divisor<float> divisor_whole(float k2) {
+  return {k2, __frcp_rn(k2)};
+}
+__device__ __forceinline__ Divisor<double> divisor_whole(double k2) { return {k2, 1.0 / k2}; }
+// den >= 1 in FP64.  FP32: one Newton step in FP64 from the FP32 reciprocal
+// (relative error about 2^-46 before the rounding to FP32).
+template <typename T>
+__device__ __forceinline__ Divisor<T> divisor_of(double den) {
+  if constexpr (sizeof(T) == 8) {
+    return {den, 1.0 / den};
+  } else {
+    const double r0 = (double)__frcp_rn((float)den);
+    return {(T)den, (T)fma_rn(fma_rn(-den, r0, 1.0), r0, r0)};
+  }
+}
+
 // Field f of the update's z-forward: the cross product (f < 3) or, with the
 // eddy stress, tau_{f-3}; selected with constant indices.
 __device__ __forceinline__ const void* update_field(const UpdateArgs& a, int f) {
@@ -631,7 +672,6 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
   const int RS = tile_stride(L, W, (int)sizeof(C));
   const int64_t nxy = (int64_t)a.nx * a.ny;
   const int64_t base = blk * W;
-  const int per = W * L;
 
   // thread t owns z line (field, base + w) at positions j + e*TPL with
   // w = t mod W, j = (t / W) mod TPL, field = t / (W*TPL): consecutive threads
@@ -654,28 +694,62 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
       for (int e = 0; e < E; e++) row[pad_pos(j + TPL * e)] = v[e];
     }
   }
-  __syncthreads();
-
+  // The update.  W is a power of two that divides the thread count, so a thread
+  // keeps one (x, y) column of the tile and walks down z: kx, ky and the
+  // pointer step are loop constants (dividing the flat point index by the
+  // run-time W cost more instructions than the update's arithmetic).  The
+  // loads of the next point are issued before the current one is computed, the
+  // first ones before the rows' barrier.
   const T hK = (T)a.hK, nuhK = (T)a.nuhK;
-  double s_div = 0, s_e = 0, s_w = 0, m_div = 0;
+  double s_div = 0, s_e = 0, s_w = 0;
+  T m_div = 0;  // the FP64 maximum of FP32 values is one of them
   C* __restrict__ Vp[3] = {reinterpret_cast<C*>(a.V[0]), reinterpret_cast<C*>(a.V[1]),
                            reinterpret_cast<C*>(a.V[2])};
   C* __restrict__ Cp[3] = {reinterpret_cast<C*>(a.C0[0]), reinterpret_cast<C*>(a.C0[1]),
                            reinterpret_cast<C*>(a.C0[2])};
-  auto update_point = [&](int q, const C (&V1)[3], const C (&c0)[3]) {
-    const int w = q % W, z = q / W;
-    const int64_t xy = base + w;
-    const int x = (int)(xy & (a.nx - 1)), y = (int)(xy >> a.lx);
-    const int64_t idx = xy + nxy * z;
-    const T kx = a.kx_half ? (T)x : (T)freq_i(x, a.nx);
-    const T ky = (T)freq_i(y, a.ny), kz = (T)freq_i(z, a.nz);
-    const double k2d = (double)kx * kx + (double)ky * ky + (double)kz * kz;
+  const int w = threadIdx.x & (W - 1), wsh = 31 - __clz(W);
+  const int dz = nthr >> wsh;
+  const int64_t xy = base + w;
+  const int x = (int)(xy & (a.nx - 1)), y = (int)(xy >> a.lx);
+  const T kx = a.kx_half ? (T)x : (T)freq_i(x, a.nx);
+  const T ky = (T)freq_i(y, a.ny);
+  const T kxy2 = kx * kx + ky * ky;  // whole numbers: exact in T
+  const bool line_nyq = y == (a.ny >> 1) || (!a.kx_half && x == (a.nx >> 1));
+  // half spectrum: each stored kx > 0 mode stands for itself and its conjugate
+  const double wgt = (a.kx_half && x > 0) ? 2.0 : 1.0;
+  int z = threadIdx.x >> wsh;
+  int64_t idx = xy + nxy * z;
+  const int64_t didx = nxy * dz;
+  C V1n[3], c0n[3];
+  if (z < L) {
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      V1n[d] = Vp[d][idx];
+      c0n[d] = Cp[d][idx];
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (; z < L; z += dz, idx += didx) {
+    C V1[3], c0[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      V1[d] = V1n[d];
+      c0[d] = c0n[d];
+    }
+    if (z + dz < L) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        V1n[d] = Vp[d][idx + didx];
+        c0n[d] = Cp[d][idx + didx];
+      }
+    }
+    const T kz = (T)freq_i(z, a.nz);
+    const T k2 = fma_rn(kz, kz, kxy2);
+    const double k2d = (double)k2;
     // modes beyond the cutoff are not evolved (zero velocity and history)
     const bool cut = k2d > a.kc2;
-    const bool nyq = cut || y == (a.ny >> 1) || (!a.kx_half && x == (a.nx >> 1)) ||
-                     z == (a.nz >> 1);
-    // half spectrum: each stored kx > 0 mode stands for itself and its conjugate
-    const double wgt = (a.kx_half && x > 0) ? 2.0 : 1.0;
+    const bool nyq = cut || line_nyq || z == (a.nz >> 1);
     C c1[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) c1[d] = nyq ? mk((T)0, (T)0) : sm[(d * W + w) * RS + pad_pos(z)];
@@ -695,82 +769,48 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
       }
     }
     const T kk[3] = {kx, ky, kz};
-    const T k2 = kx * kx + ky * ky + kz * kz;
-    // F = K/2 (3 c1 - c0)                      (ns.cpp:171)
-    // lap1 = nu K/2 (-|k|^2 V1)                (ns.cpp:174)
-    // s = V1 + lap1 + F; G = div s / (-|k|^2)  (ns.cpp:177-178)
-    C F[3], lap[3], s[3];
+    // F = K/2 (3 c1 - c0)                          (ns.cpp:171)
+    // lap1 = nu K/2 (-|k|^2 V1)                    (ns.cpp:174)
+    // s = V1 + lap1 + F; G = div s / (-|k|^2)      (ns.cpp:177-178)
+    // Vhalf = V1 + F - grad G; V = (Vhalf + lap1) / (1 + nu K/2 |k|^2)
+    //   = (s - k (k . s) / |k|^2) / (1 + nu K/2 |k|^2)   (ns.cpp:181-187)
+    const T lc = -mul_rn(nuhK, k2);
+    C s[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      F[d] = cscale(hK, csub(cscale((T)3, c1[d]), c0[d]));
-      lap[d] = cscale(nuhK, cscale(-k2, V1[d]));
-      s[d] = cadd(cadd(V1[d], lap[d]), F[d]);
+      s[d].x = fma_rn(hK, fma_rn((T)3, c1[d].x, -c0[d].x), fma_rn(lc, V1[d].x, V1[d].x));
+      s[d].y = fma_rn(hK, fma_rn((T)3, c1[d].y, -c0[d].y), fma_rn(lc, V1[d].y, V1[d].y));
     }
-    C G = cadd(cadd(ikmul(kx, s[0]), ikmul(ky, s[1])), ikmul(kz, s[2]));
-    // The divisors -|k|^2 (projection) and 1 + nu K/2 |k|^2 (Crank-Nicolson)
-    // are formed in FP64.  complex128 divides as the reference does; complex64
-    // multiplies by the FP64 reciprocals rounded once to FP32.
-    const bool nonzero = k2d != 0.0;
-    const double den_cn = 1.0 + a.nuhK * k2d;
-    T r_p = (T)1, r_cn = (T)1;
-    if constexpr (sizeof(T) == 4) {
-      if (nonzero) {
-        r_p = (T)(-1.0 / k2d);
-        r_cn = (T)(1.0 / den_cn);
-      }
-      G = cscale(r_p, G);
-    } else {
-      if (nonzero) G = mk(G.x / -k2d, G.y / -k2d);
-    }
-    // Vhalf = V1 + F - grad G; V = (Vhalf + lap1) / (1 + nu K/2 |k|^2)  (ns.cpp:181-187)
+    C g = mk(fma_rn(kz, s[2].x, fma_rn(ky, s[1].x, mul_rn(kx, s[0].x))),
+             fma_rn(kz, s[2].y, fma_rn(ky, s[1].y, mul_rn(kx, s[0].y))));
+    // the divisors |k|^2 (projection) and 1 + nu K/2 |k|^2 (Crank-Nicolson),
+    // the latter formed in FP64
+    const Divisor<T> by_k2 = divisor_whole(k2);
+    const Divisor<T> by_cn = divisor_of<T>(fma_rn(a.nuhK, k2d, 1.0));
+    g = k2 != (T)0 ? mk(by_k2.under(g.x), by_k2.under(g.y)) : mk((T)0, (T)0);
     C Vn[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      C vh = csub(cadd(V1[d], F[d]), ikmul(kk[d], G));
-      C vv = cadd(vh, lap[d]);
-      if constexpr (sizeof(T) == 4) {
-        vv = cscale(r_cn, vv);
-      } else {
-        if (nonzero) vv = mk(vv.x / den_cn, vv.y / den_cn);
-      }
+      C vv = mk(by_cn.under(fma_rn(-kk[d], g.x, s[d].x)), by_cn.under(fma_rn(-kk[d], g.y, s[d].y)));
       if (cut) vv = mk((T)0, (T)0);
       Vn[d] = vv;
       Vp[d][idx] = vv;
       Cp[d][idx] = c1[d];
       if constexpr (KEEP) sm[(d * W + w) * RS + pad_pos(z)] = vv;
     }
-    // diagnostics of the new velocity: per-mode terms in T, sums in FP64
-    const C dv = cadd(cadd(ikmul(kx, Vn[0]), ikmul(ky, Vn[1])), ikmul(kz, Vn[2]));
-    const double ad = (double)sqrt(dv.x * dv.x + dv.y * dv.y);
-    s_div += wgt * ad;
+    // diagnostics of the new velocity: per-mode terms in T, sums in FP64;
+    // |k x V|^2 = |k|^2 |V|^2 - |k . V|^2
+    const T dx = fma_rn(kz, Vn[2].x, fma_rn(ky, Vn[1].x, mul_rn(kx, Vn[0].x)));
+    const T dy = fma_rn(kz, Vn[2].y, fma_rn(ky, Vn[1].y, mul_rn(kx, Vn[0].y)));
+    const T d2 = fma_rn(dx, dx, mul_rn(dy, dy));
+    const T ad = sqrt(d2);
+    s_div = fma_rn(wgt, (double)ad, s_div);
     m_div = fmax(m_div, ad);
     T e2 = 0;
 #pragma unroll
-    for (int d = 0; d < 3; d++) e2 += Vn[d].x * Vn[d].x + Vn[d].y * Vn[d].y;
-    const C om0 = csub(ikmul(ky, Vn[2]), ikmul(kz, Vn[1]));
-    const C om1 = csub(ikmul(kz, Vn[0]), ikmul(kx, Vn[2]));
-    const C om2 = csub(ikmul(kx, Vn[1]), ikmul(ky, Vn[0]));
-    const T w2 = om0.x * om0.x + om0.y * om0.y + om1.x * om1.x + om1.y * om1.y +
-                 om2.x * om2.x + om2.y * om2.y;
-    s_e += wgt * (double)e2;
-    s_w += wgt * (double)w2;
-  };
-  // two points per iteration: the 12 global loads of both are issued first
-  for (int q0 = threadIdx.x; q0 < per; q0 += 2 * nthr) {
-    const int q1 = q0 + nthr;
-    const bool has1 = q1 < per;
-    C V1a[3], c0a[3], V1b[3], c0b[3];
-    const int64_t ia = base + (q0 % W) + nxy * (q0 / W);
-    const int64_t ib = has1 ? base + (q1 % W) + nxy * (q1 / W) : ia;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      V1a[d] = Vp[d][ia];
-      c0a[d] = Cp[d][ia];
-      V1b[d] = Vp[d][ib];
-      c0b[d] = Cp[d][ib];
-    }
-    update_point(q0, V1a, c0a);
-    if (has1) update_point(q1, V1b, c0b);
+    for (int d = 0; d < 3; d++) e2 = fma_rn(Vn[d].x, Vn[d].x, fma_rn(Vn[d].y, Vn[d].y, e2));
+    s_e = fma_rn(wgt, (double)e2, s_e);
+    s_w = fma_rn(wgt, (double)fma_rn(k2, e2, -d2), s_w);
   }
   // block reduction of the diagnostics
   for (int o = 16; o > 0; o >>= 1) {
@@ -784,7 +824,7 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
     red[0][warp] = s_div;
     red[1][warp] = s_e;
     red[2][warp] = s_w;
-    red[3][warp] = m_div;
+    red[3][warp] = (double)m_div;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -912,11 +952,11 @@ __device__ __forceinline__ void zfwd_update_curl_tile(const UpdateArgs& a,
       const C va = RELOAD ? ga[idx0 + e * step] : pa[pad_pos(p)];
       const C vb = RELOAD ? gb[idx0 + e * step] : pb[pad_pos(p)];
       if (d == 0)
-        v[e] = csub(ikmul(ky, va), ikmul(kz, vb));
+        v[e] = curl_part(ky, va, kz, vb);
       else if (d == 1)
-        v[e] = csub(ikmul(kz, va), ikmul(kx, vb));
+        v[e] = curl_part(kz, va, kx, vb);
       else
-        v[e] = csub(ikmul(kx, va), ikmul(ky, vb));
+        v[e] = curl_part(kx, va, ky, vb);
     }
   }
   // the last stage of the first transform read its exchange row before a
