@@ -269,6 +269,11 @@ bool vec_ok(const void* const v[3], const char* what) {
 
 using namespace sns;
 
+// Steps in one graph for boxes that fit L2: between two graph launches the GPU
+// idles for about 2 us, which a step of such a box (10 to 100 us) feels.  B200,
+// complex64: 32^3 14.8 -> 12.4 us a step, 64^3 31.2 -> 29.7 us.
+constexpr int kBatchSteps = 8;
+
 // ---- stepper object ----------------------------------------------------------
 struct sns_ns {
   NSPlan pl;
@@ -299,6 +304,9 @@ struct sns_ns {
   cudaStream_t cap = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  // kBatchSteps steps in one graph, for boxes whose step is a few microseconds
+  cudaGraph_t batch_graph = nullptr;
+  cudaGraphExec_t batch = nullptr;
 };
 
 namespace {
@@ -308,6 +316,10 @@ void drop_graph(sns_ns* h) {
   if (h->graph) cudaGraphDestroy(h->graph);
   h->exec = nullptr;
   h->graph = nullptr;
+  if (h->batch) cudaGraphExecDestroy(h->batch);
+  if (h->batch_graph) cudaGraphDestroy(h->batch_graph);
+  h->batch = nullptr;
+  h->batch_graph = nullptr;
 }
 
 // One step (plain or closure) queued on `s`.
@@ -325,7 +337,7 @@ int step_on(sns_ns* h, cudaStream_t s, cudaEvent_t* ev) {
                       ev, h->W, &h->carried);
 }
 
-int capture_step(sns_ns* h) {
+int capture_steps(sns_ns* h, int steps, cudaGraph_t* graph, cudaGraphExec_t* exec) {
   int rc = OK;
   if (!h->cap)
     rc = cuda_status(cudaStreamCreateWithFlags(&h->cap, cudaStreamNonBlocking),
@@ -334,19 +346,20 @@ int capture_step(sns_ns* h) {
   if ((rc = cuda_status(cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal),
                         "sns_ns_step(capture)")))
     return rc;
-  const int src = step_on(h, h->cap, nullptr);
+  int src = OK;
+  for (int t = 0; t < steps && !src; t++) src = step_on(h, h->cap, nullptr);
   cudaGraph_t g = nullptr;
   rc = cuda_status(cudaStreamEndCapture(h->cap, &g), "sns_ns_step(capture)");
   if (src || rc) {
     if (g) cudaGraphDestroy(g);
     return src ? src : rc;
   }
-  if ((rc = cuda_status(cudaGraphInstantiate(&h->exec, g, 0), "sns_ns_step(instantiate)"))) {
+  if ((rc = cuda_status(cudaGraphInstantiate(exec, g, 0), "sns_ns_step(instantiate)"))) {
     cudaGraphDestroy(g);
-    h->exec = nullptr;
+    *exec = nullptr;
     return rc;
   }
-  h->graph = g;
+  *graph = g;
   return OK;
 }
 
@@ -812,7 +825,10 @@ int sns_ns_step(sns_ns* h, int nsteps) {
     return ERR_ARG;
   }
   if (!h->profiling) {
-    for (int t = 0; t < nsteps; t++) {
+    // (a closure step's launches overlap their neighbours' edges, which measured
+    // slower across steps: 72 -> 79 us a 64^3 step)
+    const bool small = h->cl.model == CLOSURE_NONE && ns_fits_l2(h->pl);
+    for (int t = 0; t < nsteps;) {
       int rc = OK;
       // a captured step of a carrying plan starts from K1's output in U:
       // make it there first if the state was set since
@@ -821,13 +837,19 @@ int sns_ns_step(sns_ns* h, int nsteps) {
         if ((rc = ns_k1_once(h->pl, h->V, h->U, h->sync_words, h->s))) return rc;
         h->carried = true;
       }
-      if (h->use_graph && h->eager_done && !h->exec) rc = capture_step(h);
-      if (rc) return rc;
-      if (h->exec) {
-        rc = cuda_status(cudaGraphLaunch(h->exec, h->s), "sns_ns_step(graph)");
+      const bool whole = small && nsteps - t >= kBatchSteps;
+      if (h->use_graph && h->eager_done) {
+        if (whole && !h->batch)
+          rc = capture_steps(h, kBatchSteps, &h->batch_graph, &h->batch);
+        else if (!whole && !h->exec)
+          rc = capture_steps(h, 1, &h->graph, &h->exec);
+        if (rc) return rc;
+        rc = cuda_status(cudaGraphLaunch(whole ? h->batch : h->exec, h->s), "sns_ns_step(graph)");
+        t += whole ? kBatchSteps : 1;
       } else {
         rc = step_on(h, h->s, nullptr);
         h->eager_done = true;
+        t++;
       }
       if (rc) return rc;
       h->stepped = true;
@@ -1077,7 +1099,7 @@ int sns_ns_tune(sns_ns* h) {
 int sns_ns_describe(sns_ns* h, char* buf, int len) {
   if (!nonnull(h, "sns_ns_describe")) return ERR_ARG;
   const NSPlan& p = h->pl;
-  const char* xy = p.use_xyc ? "cluster" : p.use_xy ? "dataflow"
+  const char* xy = p.plane ? "plane" : p.use_xyc ? "cluster" : p.use_xy ? "dataflow"
                    : (p.xy_chunk > 0 && p.xy_chunk < p.nz) ? "slabs" : "separate";
   char tmp[256];
   const char* ord[3] = {"16-first", "remainder-first", "radix-8"};

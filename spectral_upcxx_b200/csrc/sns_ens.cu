@@ -608,7 +608,7 @@ int sns_ens_create(sns_ens** handle, int nboxes, const int64_t* dims, const doub
     ch.nz = std::get<2>(it->first);
     ch.box0 = (int)e->boxes.size();
     ch.nboxes = (int)it->second.size();
-    if (!rc) rc = ns_plan(ch.seq, (int)ch.nx, (int)ch.ny, (int)ch.nz, prec);
+    if (!rc) rc = ns_plan(ch.seq, (int)ch.nx, (int)ch.ny, (int)ch.nz, prec, 0, 0, false, true);
     ch.seq.use_xy = false;
     ch.seq.use_xyc = false;
     ch.seq.k1_lines = false;

@@ -32,9 +32,9 @@ __host__ __device__ constexpr int row_stride(int L) {
 // for runs of W adjacent lines (thread index w fastest; W = 1 for single x
 // lines), so its P lanes fall on distinct element slots (modulo P) when the
 // stride is J times an odd number.  J = 1 is an odd stride.
-__host__ __device__ constexpr int tile_stride(int L, int W, int esz = 8) {
+__host__ __device__ constexpr int tile_stride(int L, int W, int esz = 8, int E = 16) {
   const int P = 128 / esz;
-  const int tpl = L >= 16 ? L / 16 : 1;
+  const int tpl = L >= E ? L / E : 1;
   const int J = W >= P ? 1 : (P / W < tpl ? P / W : tpl);
   int rs = pad_pos(L);
   if (J >= P) return rs;
@@ -42,7 +42,9 @@ __host__ __device__ constexpr int tile_stride(int L, int W, int esz = 8) {
   return rs;
 }
 // Tiles of x lines.
-__host__ __device__ constexpr int xrow_stride(int L, int esz = 8) { return tile_stride(L, 1, esz); }
+__host__ __device__ constexpr int xrow_stride(int L, int esz = 8, int E = 16) {
+  return tile_stride(L, 1, esz, E);
+}
 
 // Radix orders of a line (all give the same transform to rounding; the
 // autotuner picks one per line length):
@@ -51,11 +53,16 @@ __host__ __device__ constexpr int xrow_stride(int L, int esz = 8) { return tile_
 //   RADIX8  radix-8 stages, the remainder (2 or 4) last
 enum RadixOrder : int { RADIX16_FIRST = 0, RADIX_REM_FIRST = 1, RADIX8 = 2, kRadixOrders = 3 };
 
-template <int L, int ORD = RADIX16_FIRST>
+//
+// EM is the elements per thread of lines of at least EM: 16 for passes that
+// stream (the fewest exchanges), 8 or 4 (radix-8 or radix-4 stages whatever
+// ORD) where a few short lines leave the SMs waiting on one warp's chain.
+template <int L, int ORD = RADIX16_FIRST, int EM = 16>
 struct LinePlan {
-  static constexpr int E = (L >= 16) ? 16 : L;  // elements per thread
+  static constexpr int E = (L >= EM) ? EM : L;  // elements per thread
   static constexpr int TPL = L / E;             // threads per line
-  static constexpr int BIG = (ORD == RADIX8 && L >= 8) ? 8 : 16;  // the repeated radix
+  static constexpr int BIG =                    // the repeated radix
+      EM < 16 ? EM : (ORD == RADIX8 && L >= 8) ? 8 : 16;
   static constexpr int REM = [] {
     int r = L;
     while (r >= BIG && r % BIG == 0) r /= BIG;
@@ -160,10 +167,11 @@ __device__ __forceinline__ void line_sync() {
 // twiddle table, sg = -1 forward, +1 inverse; `sync()` synchronises the
 // threads that share the line.  The first stage writes the line's slots at
 // once, so the caller synchronises the line after its own reads of them.
-template <int L, int ORD = RADIX16_FIRST, typename C, typename T, typename Idx, typename Sync>
-__device__ __forceinline__ void line_fft_at(C (&v)[LinePlan<L>::E], C* base, Idx idx, int j,
-                                            const C* __restrict__ tw, T sg, Sync sync) {
-  using P = LinePlan<L, ORD>;
+template <int L, int ORD = RADIX16_FIRST, int EM = 16, typename C, typename T, typename Idx,
+          typename Sync>
+__device__ __forceinline__ void line_fft_at(C (&v)[LinePlan<L, ORD, EM>::E], C* base, Idx idx,
+                                            int j, const C* __restrict__ tw, T sg, Sync sync) {
+  using P = LinePlan<L, ORD, EM>;
   constexpr int E = P::E, TPL = P::TPL;
   int Ns = 1;
 #pragma unroll
@@ -222,15 +230,15 @@ __device__ __forceinline__ void line_fft_at(C (&v)[LinePlan<L>::E], C* base, Idx
 // the block must call this (it may synchronise the block when TPL > 32).
 // BLOCK = true synchronises the whole block between stages, for layouts in
 // which the threads of a line are not confined to one warp.
-template <int L, bool BLOCK = false, int ORD = RADIX16_FIRST, typename C, typename T>
-__device__ __forceinline__ void line_fft(C (&v)[LinePlan<L>::E], C* row, int j,
+template <int L, bool BLOCK = false, int ORD = RADIX16_FIRST, int EM = 16, typename C, typename T>
+__device__ __forceinline__ void line_fft(C (&v)[LinePlan<L, ORD, EM>::E], C* row, int j,
                                          const C* __restrict__ tw, T sg) {
-  line_fft_at<L, ORD>(
+  line_fft_at<L, ORD, EM>(
       v, row, [](int p) { return pad_pos(p); }, j, tw, sg, [] {
         if constexpr (BLOCK)
           __syncthreads();
         else
-          line_sync<LinePlan<L>::TPL>();
+          line_sync<LinePlan<L, ORD, EM>::TPL>();
       });
 }
 

@@ -76,9 +76,28 @@ int elems(int L) { return L >= 16 ? 16 : L; }
 
 constexpr double kL2Bytes = 126e6;  // L2 of the B200
 
+// Whether the xy phase runs as one CTA per plane: where the plane fits
+// (SNS_PLANE=0: never), unless a form of the separate passes is asked for.
+bool plane_wanted(int nx, int ny, int prec) {
+  if (const char* e = getenv("SNS_PLANE"))
+    if (e[0] == '0') return false;
+  for (const char* v : {"SNS_K1_TMA", "SNS_K1_RELOAD", "SNS_K1_SPLIT", "SNS_K1_LINES",
+                        "SNS_K1_SMEM_KB", "SNS_X_TMA", "SNS_X_OCC", "SNS_Y_TMA", "SNS_LINE_W",
+                        "SNS_RADIX_ORDER", "SNS_Z_TMA", "SNS_Z_W", "SNS_Z_PFSELF", "SNS_CARRY",
+                        "SNS_PF", "SNS_XY_PASSES", "SNS_XY_CHUNK", "SNS_XYC"})
+    if (getenv(v)) return false;
+  return plane_supported(nx, ny, prec);
+}
+
 }  // namespace
 
-int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, bool real) {
+bool ns_fits_l2(const NSPlan& p) {
+  const double esz = p.prec == PREC_C128 ? 16 : 8;
+  return 12.0 * esz * p.nx * p.ny * p.nz <= kL2Bytes;
+}
+
+int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, bool real,
+            bool separate) {
   pl = NSPlan{};
   pl.real = real;
   pl.nx_phys = nx;
@@ -101,7 +120,7 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
     }
   const size_t esz = prec == PREC_C128 ? 16 : 8;
   // fields beyond L2: the step streams from HBM
-  const bool big = 12.0 * esz * nx * ny * nz > kL2Bytes;
+  const bool big = !ns_fits_l2(pl);
   // K3 tile: G rows of all six fields, in CTAs of at most 192 threads
   // (complex64) or 96 (complex128): small CTAs drift apart, so one CTA's loads
   // run under another's transforms.  B200, 256^3: complex64 0.266 ms with 192
@@ -306,6 +325,23 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   }
   pl.k1lW = 0;
   pl.k1lT = 0;
+  pl.plane = !separate && plane_wanted(nx, ny, prec);
+  if (pl.plane) {
+    // two launches per step: the plane pass, and the update pass with the next
+    // step's K1 carried in it, in CTAs enough for the SMs
+    const int Wmax = prec == PREC_C128 ? 8 : 16;
+    int W = 1;
+    pl.carry = false;
+    while (W * 2 <= Wmax && nx % (W * 2) == 0 && (nx / (W * 2)) * ny >= 128) W *= 2;
+    for (; W >= 1 && !pl.carry; W /= 2)
+      if (carry_ok(pl, W, false)) {
+        pl.carry = true;
+        pl.carry_reload = false;
+        pl.zW = W;
+        pl.update_blocks = (nx / W) * ny;
+      }
+    pl.passes = 3;
+  }
   pl.kc2 = 1e300;
   pl.sgs_klo = 0;
   pl.sgs_kinv = 1e30;
@@ -353,7 +389,7 @@ int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* co
     pass++;
   };
   mark();
-  const bool lines = pl.k1_lines && W && !pl.use_xy && !pl.use_xyc;
+  const bool lines = pl.k1_lines && W && !pl.use_xy && !pl.use_xyc && !pl.plane;
   // K1 carried in the previous step's K5: U already holds its output
   const bool carry = pl.carry && carried && !lines;
   const bool have_k1 = carry && *carried;
@@ -387,6 +423,10 @@ int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* co
   } else if (pl.use_xyc) {
     // K2 + K3 + K4 as one cluster pass over each plane (sns_xyc.cu)
     if ((rc = xyc_run(U, nx, ny, nz, prec, s))) return rc;
+    mark();
+  } else if (pl.plane) {
+    // K2 + K3 + K4 with one CTA per plane (sns_plane.cu)
+    if ((rc = plane_run(U, nx, ny, nz, prec, pl.real, s))) return rc;
     mark();
   }
   // K2, K3, K4 on the planes [z0, z0 + pz): the passes treat the slab as an
@@ -443,7 +483,7 @@ int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* co
     }
     return OK;
   };
-  if (!pl.use_xy && !pl.use_xyc) {
+  if (!pl.use_xy && !pl.use_xyc && !pl.plane) {
     if (pl.xy_chunk > 0 && pl.xy_chunk < nz) {
       // slabs of xy_chunk planes, so each slab's intermediates stay in L2
       for (int z0 = 0; z0 < nz; z0 += pl.xy_chunk)
@@ -546,6 +586,7 @@ bool zw_ok(const NSPlan& p, int W, int max_blocks, bool halves = false) {
 int ns_tune_plan(NSPlan& pl, void* const V[3], void* const C0[3], void* const U[6],
                  double* stats, int max_blocks, int* sync_words, cudaStream_t s,
                  void* const* W) {
+  if (pl.plane) pl.tuned = true;  // nothing to choose: the plane pass has one form
   if (pl.passes != kNSPasses) return OK;
   cudaEvent_t ev[kNSPasses + 1];
   int rc = OK;

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include "sns_plane.cuh"
 #include "sns_xy.cuh"
 
 namespace sns {
@@ -35,6 +36,7 @@ struct NSPlan {
   int sgs_blocks;     // its CTAs (= diagnostics partials of a closure step)
   bool use_xy;        // xy phase as one persistent dataflow launch
   bool use_xyc;       // xy phase as one cluster pass over each plane (sns_xyc.cu)
+  bool plane;         // xy phase with one CTA per plane (sns_plane.cu)
   XYPlan xy;
   int xy_chunk;       // planes per slab of the separate xy passes (0 = all)
   int lineW;          // adjacent lines per tile of the y/z line passes (0 = default)
@@ -54,8 +56,11 @@ struct NSPlan {
 // zW > 0 and lineW > 0 select tuned tile widths (0 = defaults).
 // real = true: a real-field run on the half spectrum kx = 0 .. nx/2-1 (pl.nx
 // is then nx/2, the stored row length; pl.nx_phys = nx).
+// separate = true: the five separate passes whatever the box.
 int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW = 0, int lineW = 0,
-            bool real = false);
+            bool real = false, bool separate = false);
+// Whether the twelve fields of a step fit L2.
+bool ns_fits_l2(const NSPlan& pl);
 // One step in place on V (Fourier velocity) and C0 (previous cross product),
 // with six work fields U; per-block diagnostics go to `stats`
 // (4 doubles x update_blocks).

@@ -53,17 +53,24 @@ inline bool k1_tma_ok(const NSPlan& p, int W, int G, int S) {
 
 // Shared memory of K5 with K1 carried: 3 W update rows, and 3 W exchange
 // rows unless the new velocity is read back from V (reload).
-inline size_t update_carry_smem(int L, int W, size_t esz, bool reload) {
-  return (size_t)(reload ? 3 : 6) * W * tile_stride(L, W, (int)esz) * esz;
+inline size_t update_carry_smem(int L, int W, size_t esz, bool reload, int E = 16) {
+  return (size_t)(reload ? 3 : 6) * W * tile_stride(L, W, (int)esz, E) * esz;
+}
+// Elements per thread of the carrying update pass beside the plane pass: short
+// lines of small boxes in shorter chains of more threads (complex64 steps on
+// B200: 16^3 10.7 us with 16, 9.6 with 8, 8.3 with 4; 32^3 13.7, 12.4, 12.0).
+inline int carry_elems(const NSPlan& p) {
+  return !p.plane || p.nz < 16 || p.nz > 64 ? 16 : p.nz <= 32 ? 4 : 8;
 }
 
 // Whether K5 with K1 carried can run W-line tiles on the box.
 inline bool carry_ok(const NSPlan& p, int W, bool reload) {
   if (W > p.nx || p.nx % W) return false;
-  const int TPL = p.nz >= 16 ? p.nz / 16 : 1;
+  const int E = carry_elems(p);
+  const int TPL = p.nz >= E ? p.nz / E : 1;
   const size_t esz = p.prec == PREC_C128 ? 16 : 8;
   return 3 * W * TPL <= max_threads(p.prec) &&
-         update_carry_smem(p.nz, W, esz, reload) <= 220 * 1024;
+         update_carry_smem(p.nz, W, esz, reload, E) <= 220 * 1024;
 }
 
 // Shared memory of the TMA-staged K5: the stage (3 W x L boxes), 128 bytes of
@@ -196,16 +203,10 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 }
 
 // ---------------------------------------------------------------------------
-// K3 of a real-field run: rows of the half spectrum, M = nx/2 values
-// (kx = 0 .. M-1; kx = M is a Nyquist mode, zero).  Inverse: the real line u of
-// length 2M comes from one M-point complex FFT of
-//   Z[k] = (V[k] + conj V[M-k]) + i w^k (V[k] - conj V[M-k]),  w = e^{+2 pi i/2M},
-// V[M] = 0, as z[m] = u[2m] + i u[2m+1].  The cross product acts on the two real
-// samples of every complex slot.  Forward: Z = FFT_M(c[2m] + i c[2m+1]) and
-//   C[k] = (Z[k] + conj Z[M-k]) / 2 - i W^k (Z[k] - conj Z[M-k]) / 2,  W = e^{-2 pi i/2M}.
-// twN: the 2M-point table exp(-2 pi i m / 2M); twM: the M-point table.
-// The pre- and post-processing run on pairs (k, M-k) in shared memory, so no
-// line values stay in registers across them; FP32 fits two CTAs per SM.
+// K3 of a real-field run (r2c_rows_pre, r2c_rows_post in sns_tiles.cuh).  twN:
+// the 2M-point table exp(-2 pi i m / 2M); twM: the M-point table.  No line
+// values stay in registers across the pre- and post-processing; FP32 fits two
+// CTAs per SM.
 template <typename T, int M>
 __global__ void __launch_bounds__(384, sizeof(T) == 4 ? 2 : 1)
     k_xcross_r2c(FieldPtrs f, const cx_t<T>* __restrict__ twN, const cx_t<T>* __restrict__ twM,
@@ -233,21 +234,7 @@ __global__ void __launch_bounds__(384, sizeof(T) == 4 ? 2 : 1)
 #pragma unroll
   for (int e = 0; e < E; e++) row[pad_pos(j + TPL * e)] = v[e];
   line_sync<TPL>();
-  // Z in place, one thread per pair (k, M-k):  with A = V[k] + conj V[M-k] and
-  // B = V[k] - conj V[M-k],  Z[k] = A + i w^k B  and  Z[M-k] = conj(A - i w^k B)
-#pragma unroll 1
-  for (int e = 0; e <= M / (2 * TPL); e++) {
-    const int k = j + TPL * e;
-    if (k <= M / 2) {
-      const C vk = row[pad_pos(k)];
-      const C vm = k == 0 ? mk((T)0, (T)0) : row[pad_pos(M - k)];
-      const C vmc = mk(vm.x, -vm.y);
-      const C a = cadd(vk, vmc), b = csub(vk, vmc);
-      const C wb = cmul(mk(twN[k].x, -twN[k].y), b);  // w^k b, w = e^{+2 pi i / 2M}
-      row[pad_pos(k)] = mk(a.x - wb.y, a.y + wb.x);
-      if (k > 0 && k < M / 2) row[pad_pos(M - k)] = mk(a.x + wb.y, wb.x - a.y);
-    }
-  }
+  r2c_rows_pre<M>(row, j, twN);
   line_sync<TPL>();
 #pragma unroll
   for (int e = 0; e < E; e++) v[e] = row[pad_pos(j + TPL * e)];
@@ -266,12 +253,10 @@ __global__ void __launch_bounds__(384, sizeof(T) == 4 ? 2 : 1)
       u[d] = sm[(d * G + g) * RS + pad_pos(p)];
       w[d] = sm[((3 + d) * G + g) * RS + pad_pos(p)];
     }
-    const C c0 = mk(u[1].x * w[2].x - u[2].x * w[1].x, u[1].y * w[2].y - u[2].y * w[1].y);
-    const C c1 = mk(u[2].x * w[0].x - u[0].x * w[2].x, u[2].y * w[0].y - u[0].y * w[2].y);
-    const C c2 = mk(u[0].x * w[1].x - u[1].x * w[0].x, u[0].y * w[1].y - u[1].y * w[0].y);
-    sm[(0 * G + g) * RS + pad_pos(p)] = cscale(scale2, c0);
-    sm[(1 * G + g) * RS + pad_pos(p)] = cscale(scale2, c1);
-    sm[(2 * G + g) * RS + pad_pos(p)] = cscale(scale2, c2);
+    C c[3];
+    cross_point<true>(u, w, scale2, c);
+#pragma unroll
+    for (int d = 0; d < 3; d++) sm[(d * G + g) * RS + pad_pos(p)] = c[d];
   }
   __syncthreads();
 
@@ -288,23 +273,8 @@ __global__ void __launch_bounds__(384, sizeof(T) == 4 ? 2 : 1)
     line_sync<TPL>();
   }
   if (fld < 3) {
-    // one thread per pair (k, M-k):  with Ev = (Z[k] + conj Z[M-k]) / 2 and
-    // Od = (Z[k] - conj Z[M-k]) / 2,  C[k] = Ev - i W^k Od  and
-    // C[M-k] = conj(Ev + i W^k Od)
     C* __restrict__ dst = reinterpret_cast<C*>(select_ptr(f.out, fld)) + (row0 + gl) * M;
-#pragma unroll 1
-    for (int e = 0; e <= M / (2 * TPL); e++) {
-      const int k = j + TPL * e;
-      if (k <= M / 2) {
-        const C z = row[pad_pos(k)];
-        const C zm = row[pad_pos(k == 0 ? 0 : M - k)];
-        const C ev = mk((T)0.5 * (z.x + zm.x), (T)0.5 * (z.y - zm.y));
-        const C od = mk((T)0.5 * (z.x - zm.x), (T)0.5 * (z.y + zm.y));
-        const C wo = cmul(twN[k], od);  // W^k od
-        dst[k] = mk(ev.x + wo.y, ev.y - wo.x);
-        if (k > 0 && k < M / 2) dst[M - k] = mk(ev.x - wo.y, -(ev.y + wo.x));
-      }
-    }
+    r2c_rows_post<M>(row, j, twN, [&](int k, C c) { dst[k] = c; });
   }
 }
 
@@ -445,14 +415,14 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 
 // K5 with the next step's K1 carried in it (zfwd_update_curl_tile): the
 // update, then the z-inverse of the new V and of i k x V into a.Uo.
-template <typename T, int L, bool RELOAD>
+template <typename T, int L, bool RELOAD, int EM = 16>
 __global__ void __launch_bounds__(MaxThreads<T>::value)
     k_zfwd_update_curl(const UpdateArgs a, const cx_t<T>* __restrict__ tw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[4][32];
   pdl_trigger();
   pdl_wait();
-  zfwd_update_curl_tile<T, L, RELOAD>(a, tw, (int64_t)blockIdx.x, (int)blockDim.x,
+  zfwd_update_curl_tile<T, L, RELOAD, EM>(a, tw, (int64_t)blockIdx.x, (int)blockDim.x,
                                       reinterpret_cast<cx_t<T>*>(smem_raw), red);
 }
 
@@ -813,12 +783,12 @@ int launch_update(const NSPlan& pl, const UpdateArgs& a, cudaStream_t s) {
   return OK;
 }
 
-template <typename T, int L, bool RELOAD>
+template <typename T, int L, bool RELOAD, int EM = 16>
 int launch_update_carry(const NSPlan& pl, const UpdateArgs& a, cudaStream_t s) {
   using C = cx_t<T>;
-  constexpr int TPL = LinePlan<L>::TPL;
+  constexpr int TPL = LinePlan<L, RADIX16_FIRST, EM>::TPL;
   const int threads = 3 * a.W * TPL;
-  const size_t smem = update_carry_smem(L, a.W, sizeof(C), RELOAD);
+  const size_t smem = update_carry_smem(L, a.W, sizeof(C), RELOAD, EM);
   const int blocks = (int)(((int64_t)pl.nx * pl.ny) / a.W);
   if (a.W > pl.nx || pl.nx % a.W || threads > MaxThreads<T>::value) {
     set_error("K5 with K1 carried: the tile width does not fit the box");
@@ -828,16 +798,16 @@ int launch_update_carry(const NSPlan& pl, const UpdateArgs& a, cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr[dev & 63]) {
-    cudaError_t e = allow_max_dynamic_smem(k_zfwd_update_curl<T, L, RELOAD>);
+    cudaError_t e = allow_max_dynamic_smem(k_zfwd_update_curl<T, L, RELOAD, EM>);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(k_zfwd_update_curl)");
     attr[dev & 63] = true;
   }
   const C* tw = reinterpret_cast<const C*>(twiddles(L, sizeof(T) == 8 ? PREC_C128 : PREC_C64));
   UpdateArgs ap = a;
-  ap.pf = tiles_in_waves(k_zfwd_update_curl<T, L, RELOAD>, threads, smem, pl.pf_waves);
+  ap.pf = tiles_in_waves(k_zfwd_update_curl<T, L, RELOAD, EM>, threads, smem, pl.pf_waves);
   ap.pf_self = pl.z_pfself;
   cudaError_t e =
-      launch_pdl(k_zfwd_update_curl<T, L, RELOAD>, dim3(blocks), dim3(threads), smem, s, ap, tw);
+      launch_pdl(k_zfwd_update_curl<T, L, RELOAD, EM>, dim3(blocks), dim3(threads), smem, s, ap, tw);
   if (e != cudaSuccess) return cuda_status(e, "k_zfwd_update_curl");
   return OK;
 }
@@ -965,6 +935,10 @@ int ns_update_carry(const NSPlan& pl, const UpdateArgs& a, cudaStream_t s) {
   switch (pl.nz) {
 #define SNS_CARRY_CASE(L)                                                                    \
   case L:                                                                                    \
+    if constexpr (L >= 16 && L <= 64) {                                                      \
+      constexpr int EM = L <= 32 ? 4 : 8;                                                    \
+      if (!r && carry_elems(pl) == EM) return launch_update_carry<T, L, false, EM>(pl, a, s); \
+    }                                                                                        \
     return r ? launch_update_carry<T, L, true>(pl, a, s) : launch_update_carry<T, L, false>(pl, a, s);
     SNS_CARRY_CASE(4)
     SNS_CARRY_CASE(8)

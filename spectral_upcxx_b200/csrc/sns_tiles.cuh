@@ -477,6 +477,77 @@ __device__ __forceinline__ void curl_zpass_tile_staged(const LineGeo& geo, const
   }
 }
 
+// Point of the cross product c = scale2 (u x w): complex values, or (REAL) two
+// real samples per slot.
+template <bool REAL, typename C, typename T>
+__device__ __forceinline__ void cross_point(const C (&u)[3], const C (&w)[3], T scale2,
+                                            C (&c)[3]) {
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const C &ua = u[(d + 1) % 3], &ub = u[(d + 2) % 3];
+    const C &wa = w[(d + 1) % 3], &wb = w[(d + 2) % 3];
+    const C p = REAL ? mk(fma_rn(ua.x, wb.x, -mul_rn(ub.x, wa.x)),
+                          fma_rn(ua.y, wb.y, -mul_rn(ub.y, wa.y)))
+                     : csub(cmul(ua, wb), cmul(ub, wa));
+    c[d] = mk(mul_rn(scale2, p.x), mul_rn(scale2, p.y));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// K3 of a real-field run: rows of the half spectrum, M = nx/2 values
+// (kx = 0 .. M-1; kx = M is a Nyquist mode, zero).  Inverse: the real line u of
+// length 2M comes from one M-point complex FFT of
+//   Z[k] = (V[k] + conj V[M-k]) + i w^k (V[k] - conj V[M-k]),  w = e^{+2 pi i/2M},
+// V[M] = 0, as z[m] = u[2m] + i u[2m+1].  The cross product acts on the two real
+// samples of every complex slot.  Forward: Z = FFT_M(c[2m] + i c[2m+1]) and
+//   C[k] = (Z[k] + conj Z[M-k]) / 2 - i W^k (Z[k] - conj Z[M-k]) / 2,  W = e^{-2 pi i/2M}.
+// twN: the 2M-point table exp(-2 pi i m / 2M).  The pre- and post-processing run
+// on pairs (k, M-k) of a line in shared memory (padded row, thread j of TPL).
+//
+// Z in place, one thread per pair (k, M-k):  with A = V[k] + conj V[M-k] and
+// B = V[k] - conj V[M-k],  Z[k] = A + i w^k B  and  Z[M-k] = conj(A - i w^k B)
+template <int M, int TPL = LinePlan<M>::TPL, typename C>
+__device__ __forceinline__ void r2c_rows_pre(C* row, int j, const C* __restrict__ twN) {
+#pragma unroll 1
+  for (int e = 0; e <= M / (2 * TPL); e++) {
+    const int k = j + TPL * e;
+    if (k <= M / 2) {
+      const C vk = row[pad_pos(k)];
+      C vm = vk;
+      if (k == 0)
+        vm.x = vm.y = 0;
+      else
+        vm = row[pad_pos(M - k)];
+      const C vmc = mk(vm.x, -vm.y);
+      const C a = cadd(vk, vmc), b = csub(vk, vmc);
+      const C wb = cmul(mk(twN[k].x, -twN[k].y), b);  // w^k b, w = e^{+2 pi i / 2M}
+      row[pad_pos(k)] = mk(a.x - wb.y, a.y + wb.x);
+      if (k > 0 && k < M / 2) row[pad_pos(M - k)] = mk(a.x + wb.y, wb.x - a.y);
+    }
+  }
+}
+// One thread per pair (k, M-k):  with Ev = (Z[k] + conj Z[M-k]) / 2 and
+// Od = (Z[k] - conj Z[M-k]) / 2,  C[k] = Ev - i W^k Od  and
+// C[M-k] = conj(Ev + i W^k Od), handed to store(k, C[k])
+template <int M, int TPL = LinePlan<M>::TPL, typename C, typename Store>
+__device__ __forceinline__ void r2c_rows_post(const C* row, int j, const C* __restrict__ twN,
+                                              Store store) {
+  using T = decltype(row[0].x + 0);
+#pragma unroll 1
+  for (int e = 0; e <= M / (2 * TPL); e++) {
+    const int k = j + TPL * e;
+    if (k <= M / 2) {
+      const C z = row[pad_pos(k)];
+      const C zm = row[pad_pos(k == 0 ? 0 : M - k)];
+      const C ev = mk((T)0.5 * (z.x + zm.x), (T)0.5 * (z.y - zm.y));
+      const C od = mk((T)0.5 * (z.x - zm.x), (T)0.5 * (z.y + zm.y));
+      const C wo = cmul(twN[k], od);  // W^k od
+      store(k, mk(ev.x + wo.y, ev.y - wo.x));
+      if (k > 0 && k < M / 2) store(M - k, mk(ev.x - wo.y, -(ev.y + wo.x)));
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // K3 of the NS step: x lines -- inverse 6 fields, 1/N^2-scaled complex cross
 // product u x omega, forward 3 fields (src/Vector.cpp:79-89).  A tile is G
@@ -516,12 +587,10 @@ __device__ __forceinline__ void xcross_tile_from(const Fields& f, const cx_t<T>*
       u[d] = sm[(d * G + g) * RS + pad_pos(p)];
       w[d] = sm[((3 + d) * G + g) * RS + pad_pos(p)];
     }
-    const C c0 = csub(cmul(u[1], w[2]), cmul(u[2], w[1]));
-    const C c1 = csub(cmul(u[2], w[0]), cmul(u[0], w[2]));
-    const C c2 = csub(cmul(u[0], w[1]), cmul(u[1], w[0]));
-    sm[(0 * G + g) * RS + pad_pos(p)] = cscale(scale2, c0);
-    sm[(1 * G + g) * RS + pad_pos(p)] = cscale(scale2, c1);
-    sm[(2 * G + g) * RS + pad_pos(p)] = cscale(scale2, c2);
+    C c[3];
+    cross_point<false>(u, w, scale2, c);
+#pragma unroll
+    for (int d = 0; d < 3; d++) sm[(d * G + g) * RS + pad_pos(p)] = c[d];
   }
   __syncthreads();
 
@@ -659,17 +728,17 @@ __device__ __forceinline__ const void* update_field(const UpdateArgs& a, int f) 
 // (component d of line w at (d W + w) RS + pad_pos(z), where the z-forward of
 // the cross product was), ordered before the caller's reads by the block
 // barrier of the diagnostics' reduction.
-template <typename T, int L, bool SGS, bool KEEP = false, typename Load>
+template <typename T, int L, bool SGS, bool KEEP = false, int EM = 16, typename Load>
 __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
                                                       const cx_t<T>* __restrict__ tw, int64_t blk,
                                                       int nthr, cx_t<T>* sm, double (*red)[32],
                                                       Load load) {
   using C = cx_t<T>;
-  using P = LinePlan<L>;
+  using P = LinePlan<L, RADIX16_FIRST, EM>;
   constexpr int E = P::E, TPL = P::TPL;
 
   const int W = a.W;
-  const int RS = tile_stride(L, W, (int)sizeof(C));
+  const int RS = tile_stride(L, W, (int)sizeof(C), EM);
   const int64_t nxy = (int64_t)a.nx * a.ny;
   const int64_t base = blk * W;
 
@@ -689,7 +758,7 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
       C* row = sm + (fld * W + w) * RS;
       C v[E];
       load(fld, w, j, v);
-      line_fft<L, true>(v, row, j, tw, (T)-1);
+      line_fft<L, true, RADIX16_FIRST, EM>(v, row, j, tw, (T)-1);
 #pragma unroll
       for (int e = 0; e < E; e++) row[pad_pos(j + TPL * e)] = v[e];
     }
@@ -845,16 +914,17 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
 
 // K5 tile with its loads from HBM straight into registers, optionally asking
 // L2 for the inputs of tile blk + pf first.
-template <typename T, int L, bool SGS = false, bool KEEP = false>
+template <typename T, int L, bool SGS = false, bool KEEP = false, int EM = 16>
 __device__ __forceinline__ void zfwd_update_tile(const UpdateArgs& a,
                                                  const cx_t<T>* __restrict__ tw, int64_t blk,
                                                  int nthr, cx_t<T>* sm, double (*red)[32]) {
   using C = cx_t<T>;
-  constexpr int E = LinePlan<L>::E, TPL = LinePlan<L>::TPL;
+  using P = LinePlan<L, RADIX16_FIRST, EM>;
+  constexpr int E = P::E, TPL = P::TPL;
   const int W = a.W;
   const int64_t nxy = (int64_t)a.nx * a.ny;
   const int64_t base = blk * W;
-  zfwd_update_tile_from<T, L, SGS, KEEP>(a, tw, blk, nthr, sm, red, [&](int fld, int w, int j, C (&v)[E]) {
+  zfwd_update_tile_from<T, L, SGS, KEEP, EM>(a, tw, blk, nthr, sm, red, [&](int fld, int w, int j, C (&v)[E]) {
     const C* __restrict__ src = reinterpret_cast<const C*>(
         SGS ? update_field(a, fld) : (fld == 0 ? a.U[0] : fld == 1 ? a.U[1] : a.U[2]));
     const int64_t i0 = base + w + nxy * j;
@@ -902,15 +972,16 @@ __device__ __forceinline__ void zfwd_update_tile(const UpdateArgs& a,
 // written (L1/L2, not DRAM; the block barrier of the diagnostics makes the
 // stores visible), and each thread's own row serves as its exchange row, as
 // in curl_zpass_tile_reload.
-template <typename T, int L, bool RELOAD = false>
+template <typename T, int L, bool RELOAD = false, int EM = 16>
 __device__ __forceinline__ void zfwd_update_curl_tile(const UpdateArgs& a,
                                                       const cx_t<T>* __restrict__ tw, int64_t blk,
                                                       int nthr, cx_t<T>* sm, double (*red)[32]) {
   using C = cx_t<T>;
-  constexpr int E = LinePlan<L>::E, TPL = LinePlan<L>::TPL;
-  zfwd_update_tile<T, L, false, !RELOAD>(a, tw, blk, nthr, sm, red);
+  using P = LinePlan<L, RADIX16_FIRST, EM>;
+  constexpr int E = P::E, TPL = P::TPL;
+  zfwd_update_tile<T, L, false, !RELOAD, EM>(a, tw, blk, nthr, sm, red);
   const int W = a.W;
-  const int RS = tile_stride(L, W, (int)sizeof(C));
+  const int RS = tile_stride(L, W, (int)sizeof(C), EM);
   const int64_t nxy = (int64_t)a.nx * a.ny;
   const int w = threadIdx.x % W, s = threadIdx.x / W;
   const int j = s % TPL, d = s / TPL;  // line w of component d, positions j + e TPL
@@ -931,7 +1002,7 @@ __device__ __forceinline__ void zfwd_update_curl_tile(const UpdateArgs& a,
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = vr[pad_pos(j + TPL * e)];
   }
-  line_fft<L, true>(v, xrow, j, tw, (T)1);
+  line_fft<L, true, RADIX16_FIRST, EM>(v, xrow, j, tw, (T)1);
   {
     C* __restrict__ dst = reinterpret_cast<C*>(d == 0 ? a.Uo[0] : d == 1 ? a.Uo[1] : a.Uo[2]);
 #pragma unroll
@@ -961,7 +1032,7 @@ __device__ __forceinline__ void zfwd_update_curl_tile(const UpdateArgs& a,
   }
   // the last stage of the first transform read its exchange row before a
   // block barrier, so the second may write it at once
-  line_fft<L, true>(v, xrow, j, tw, (T)1);
+  line_fft<L, true, RADIX16_FIRST, EM>(v, xrow, j, tw, (T)1);
   {
     C* __restrict__ dst = reinterpret_cast<C*>(d == 0 ? a.Uo[3] : d == 1 ? a.Uo[4] : a.Uo[5]);
 #pragma unroll
