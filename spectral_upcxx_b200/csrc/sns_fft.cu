@@ -293,6 +293,51 @@ LineGeo axis_geo(int axis, int nx, int ny, int nz, int prec, int wmax, int tmax,
   return g;
 }
 
+int fft_shape(FftShape& p, int nx, int ny, int nz, int nf, int prec, const void* const* tw_axes,
+              cudaStream_t stream) {
+  p = FftShape{};
+  p.nx = nx;
+  p.ny = ny;
+  p.nz = nz;
+  p.nf = nf;
+  p.prec = prec;
+  p.tw = tw_axes;
+  // a tuned plan of this shape (callers that pass their own twiddle tables
+  // keep the default plan and never trigger a tuning run)
+  if (!tw_axes) {
+    p.tuned = fft3d_tuned(nx, ny, nz, nf, prec, &p.tc);
+    if (!p.tuned && tune_on_first_use()) {
+      int rc = fft3d_tune(nx, ny, nz, nf, prec, stream);
+      if (rc) return rc;
+      p.tuned = fft3d_tuned(nx, ny, nz, nf, prec, &p.tc);
+    }
+  }
+  // the TMA-staged form of a pass where the tuned plan chose it (SNS_FFT_TMA =
+  // 1 or 2 stages asks for it on the passes of an untuned plan)
+  if (const char* e = getenv("SNS_FFT_TMA")) p.forced = atoi(e);
+  if (p.forced != 1 && p.forced != 2) p.forced = 0;
+  p.err = (p.tuned || p.forced) && !tw_axes ? fft_tma_err_word() : nullptr;
+  return OK;
+}
+
+int fft_axis_pass(const FftShape& p, const FieldPtrs& f, int axis, int sign, int flags,
+                  double scale, cudaStream_t stream) {
+  LineGeo g = p.tuned ? axis_geo(axis, p.nx, p.ny, p.nz, p.prec, p.tc.wmax[axis], p.tc.tmax[axis],
+                                 p.tc.ord[axis])
+                      : axis_geo(axis, p.nx, p.ny, p.nz, p.prec);
+  // The y pass of a forward transform and the z and x passes of an inverse one
+  // walk their tiles from the last to the first: x and y tiles both follow the
+  // z planes, and an inverse often follows a forward transform's z pass, so
+  // each starts on what the pass before it left in L2 (256^3 complex64 forward +
+  // inverse on B200: 0.293 ms against 0.303 in plain order).
+  g.rev = (sign < 0) == (axis == 1);
+  if (p.tw) g.tw = p.tw[axis];
+  const int S = p.tuned ? p.tc.tma[axis] : p.forced;
+  if (S && p.err && f.n <= 6 && line_tma_ok(g, p.prec, S))
+    return run_line_pass_tma(g, f, sign, flags, scale, p.prec, stream, S, p.err);
+  return run_line_pass(g, f, sign, flags, scale, p.prec, stream);
+}
+
 int fft3d(void* const* fields, int nf, int nx, int ny, int nz, int sign, int flags, int prec,
           cudaStream_t stream, const void* const* tw_axes) {
   if (nx < 1 || ny < 1 || nz < 1 || nf < 1 || nf > kMaxFields) {
@@ -307,44 +352,12 @@ int fft3d(void* const* fields, int nf, int nx, int ny, int nz, int sign, int fla
   f.n = nf;
   for (int i = 0; i < nf; i++) f.in[i] = f.out[i] = fields[i];
   const double N = (double)nx * ny * nz;
-  // a tuned plan of this shape (callers that pass their own twiddle tables
-  // keep the default plan and never trigger a tuning run)
-  FftChoice tc{};
-  bool tuned = false;
-  if (!tw_axes) {
-    tuned = fft3d_tuned(nx, ny, nz, nf, prec, &tc);
-    if (!tuned && tune_on_first_use()) {
-      int rc = fft3d_tune(nx, ny, nz, nf, prec, stream);
-      if (rc) return rc;
-      tuned = fft3d_tuned(nx, ny, nz, nf, prec, &tc);
-    }
-  }
-  // The y pass of a forward transform and the z and x passes of an inverse one
-  // walk their tiles from the last to the first: x and y tiles both follow the
-  // z planes, and an inverse often follows a forward transform's z pass, so
-  // each starts on what the pass before it left in L2 (256^3 complex64 forward +
-  // inverse on B200: 0.293 ms against 0.303 in plain order).
-  auto geo = [&](int axis) {
-    LineGeo g = tuned ? axis_geo(axis, nx, ny, nz, prec, tc.wmax[axis], tc.tmax[axis],
-                                 tc.ord[axis])
-                      : axis_geo(axis, nx, ny, nz, prec);
-    g.rev = (sign < 0) == (axis == 1);
-    return g;
+  FftShape shape;
+  if (int rc = fft_shape(shape, nx, ny, nz, nf, prec, tw_axes, stream)) return rc;
+  auto pass = [&](int axis, int fl) {
+    return fft_axis_pass(shape, f, axis, sign, fl, 1.0 / N, stream);
   };
-  // a pass of the plan: the TMA-staged form where the tuned plan chose it
-  // (SNS_FFT_TMA = 1 or 2 stages asks for it on the passes of an untuned
-  // plan)
-  int forced = 0;
-  if (const char* e = getenv("SNS_FFT_TMA")) forced = atoi(e);
-  if (forced != 1 && forced != 2) forced = 0;
-  int* err_word = (tuned || forced) && !tw_axes ? fft_tma_err_word() : nullptr;
-  auto pass = [&](int axis, const LineGeo& g, int sg, int fl) {
-    const int S = tuned ? tc.tma[axis] : forced;
-    if (S && err_word && nf <= 6 && line_tma_ok(g, prec, S))
-      return run_line_pass_tma(g, f, sg, fl, 1.0 / N, prec, stream, S, err_word);
-    return run_line_pass(g, f, sg, fl, 1.0 / N, prec, stream);
-  };
-  const bool plane = tuned ? tc.plane : true;
+  const bool plane = shape.tuned ? shape.tc.plane : true;
   if (!tw_axes && plane && fft_xy_supported(nx, ny, nz, nf, prec)) {
     // two passes: xy planes and z lines (forward xy first, inverse z first),
     // the epilogue on the second
@@ -352,10 +365,10 @@ int fft3d(void* const* fields, int nf, int nx, int ny, int nz, int sign, int fla
     if (sign < 0) {
       int rc = fft_xy_pass(f, nx, nz, sign, z_pass ? 0 : flags, 1.0 / N, prec, stream);
       if (rc || !z_pass) return rc;
-      return pass(2, geo(2), sign, flags);
+      return pass(2, flags);
     }
     if (z_pass) {
-      int rc = pass(2, geo(2), sign, 0);
+      int rc = pass(2, 0);
       if (rc) return rc;
     }
     return fft_xy_pass(f, nx, nz, sign, flags, 1.0 / N, prec, stream);
@@ -368,10 +381,7 @@ int fft3d(void* const* fields, int nf, int nx, int ny, int nz, int sign, int fla
   for (int i = 0; i < 3; i++)
     if (dims[order[i]] > 1) axes[na++] = order[i];
   for (int i = 0; i < na; i++) {
-    LineGeo g = geo(axes[i]);
-    if (tw_axes) g.tw = tw_axes[axes[i]];
-    int fl = (i == na - 1) ? flags : 0;
-    int rc = pass(axes[i], g, sign, fl);
+    int rc = pass(axes[i], (i == na - 1) ? flags : 0);
     if (rc) return rc;
   }
   if (na == 0 && flags) {

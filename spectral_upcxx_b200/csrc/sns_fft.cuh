@@ -158,6 +158,21 @@ struct FftChoice {
   int tma[3];  // stages of the TMA-staged form of each axis's pass (0: direct loads)
   bool plane;
 };
+// What a 3D transform of nf fields of one shape needs to know of its plan, and
+// one pass of it along an axis (f may be out of place): the tuned or default
+// tile, the direction in which tiles are walked, the caller's twiddle tables.
+struct FftShape {
+  int nx, ny, nz, nf, prec;
+  const void* const* tw;
+  bool tuned;
+  FftChoice tc;
+  int forced;
+  int* err;
+};
+int fft_shape(FftShape& p, int nx, int ny, int nz, int nf, int prec, const void* const* tw_axes,
+              cudaStream_t stream);
+int fft_axis_pass(const FftShape& p, const FieldPtrs& f, int axis, int sign, int flags,
+                  double scale, cudaStream_t stream);
 // Error word of the transform's TMA-staged passes on the current device
 // (null if it cannot be set up), and its check: reads and clears it,
 // SNS_ERR_TIMEOUT with the error text when a pass recorded a failure.

@@ -76,6 +76,21 @@ int elems(int L) { return L >= 16 ? 16 : L; }
 
 constexpr double kL2Bytes = 126e6;  // L2 of the B200
 
+// K3 tile: G rows of all six fields, in CTAs of at most 192 threads
+// (complex64) or 96 (complex128): small CTAs drift apart, so one CTA's loads
+// run under another's transforms.  B200, 256^3: complex64 0.266 ms with 192
+// threads, 0.283 with 96 and with 384; complex128 0.598 with 96, 0.614 with
+// 192, 0.737 with 384.
+int x_tile_rows(int nx, int64_t rows, int prec) {
+  const int TPL = nx / elems(nx);
+  const size_t esz = prec == PREC_C128 ? 16 : 8;
+  int G = 1;
+  while (6 * (G * 2) * TPL <= (prec == PREC_C128 ? 96 : 192) && rows % (G * 2) == 0 &&
+         (size_t)6 * G * 2 * xrow_stride(nx, (int)esz) * esz <= 110 * 1024)
+    G *= 2;
+  return G;
+}
+
 // Whether the xy phase runs as one CTA per plane: where the plane fits
 // (SNS_PLANE=0: never), unless a form of the separate passes is asked for.
 bool plane_wanted(int nx, int ny, int prec) {
@@ -90,6 +105,23 @@ bool plane_wanted(int nx, int ny, int prec) {
 }
 
 }  // namespace
+
+int cross_xpass(void* const in[6], void* const out[3], int nx, int ny, int nz, int prec,
+                double scale2, cudaStream_t s) {
+  NSPlan pl{};
+  pl.nx = pl.nx_phys = nx;
+  pl.ny = ny;
+  pl.nz = nz;
+  pl.prec = prec;
+  pl.scale2 = scale2;
+  pl.xG = x_tile_rows(nx, (int64_t)ny * nz, prec);
+  pl.rev = true;
+  FieldPtrs f{};
+  f.n = 6;
+  for (int i = 0; i < 6; i++) f.in[i] = in[i];
+  for (int i = 0; i < 3; i++) f.out[i] = out[i];
+  return xpass(pl, f, (int64_t)ny * nz, nullptr, s);
+}
 
 bool ns_fits_l2(const NSPlan& p) {
   const double esz = p.prec == PREC_C128 ? 16 : 8;
@@ -121,17 +153,10 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   const size_t esz = prec == PREC_C128 ? 16 : 8;
   // fields beyond L2: the step streams from HBM
   const bool big = !ns_fits_l2(pl);
-  // K3 tile: G rows of all six fields, in CTAs of at most 192 threads
-  // (complex64) or 96 (complex128): small CTAs drift apart, so one CTA's loads
-  // run under another's transforms.  B200, 256^3: complex64 0.266 ms with 192
-  // threads, 0.283 with 96 and with 384; complex128 0.598 with 96, 0.614 with
-  // 192, 0.737 with 384.
   {
     const int TPL = nx / elems(nx);
-    int G = 1;
-    while (6 * (G * 2) * TPL <= (prec == PREC_C128 ? 96 : 192) && ((int64_t)ny * nz) % (G * 2) == 0 &&
-           (size_t)6 * G * 2 * xrow_stride(nx, (int)esz) * esz <= 110 * 1024)
-      G *= 2;
+    const int G = x_tile_rows(nx, (int64_t)ny * nz, prec);
+    pl.scale2 = 1.0 / (((double)pl.nx_phys * ny * nz) * ((double)pl.nx_phys * ny * nz));
     if (6 * G * TPL > max_threads(prec)) {
       set_error("fused NS step: nx too large for the x-pass tile");
       return ERR_UNSUPPORTED;
@@ -426,7 +451,7 @@ int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* co
     mark();
   } else if (pl.plane) {
     // K2 + K3 + K4 with one CTA per plane (sns_plane.cu)
-    if ((rc = plane_run(U, nx, ny, nz, prec, pl.real, s))) return rc;
+    if ((rc = plane_run(U, U, nx, ny, nz, prec, pl.real, pl.scale2, s))) return rc;
     mark();
   }
   // K2, K3, K4 on the planes [z0, z0 + pz): the passes treat the slab as an

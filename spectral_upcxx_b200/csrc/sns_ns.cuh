@@ -11,6 +11,7 @@ namespace sns {
 struct NSPlan {
   int nx, ny, nz, prec;
   int xG;             // rows per CTA of the x cross pass
+  double scale2;      // factor of the cross product (1/N^2 for unnormalised fields)
   bool x_tma;         // the x cross pass as a persistent pass over TMA-staged rows
   bool x_occ;         // its direct-load form compiled for five CTAs of <= 192 threads per SM
   bool z_tma;         // the update pass as a persistent pass over TMA-staged z lines
@@ -59,6 +60,10 @@ struct NSPlan {
 // separate = true: the five separate passes whatever the box.
 int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW = 0, int lineW = 0,
             bool real = false, bool separate = false);
+// x-inverse, cross product and x-forward of six fields (K3 alone, out of place
+// or in place): out = scale2 (in[0..2] x in[3..5]) along x.  nx in [4, 1024].
+int cross_xpass(void* const in[6], void* const out[3], int nx, int ny, int nz, int prec,
+                double scale2, cudaStream_t s);
 // Whether the twelve fields of a step fit L2.
 bool ns_fits_l2(const NSPlan& pl);
 // One step in place on V (Fourier velocity) and C0 (previous cross product),

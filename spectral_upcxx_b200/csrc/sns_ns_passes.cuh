@@ -532,10 +532,9 @@ int launch_xcross(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream
       attr_o[dev & 63] = true;
     }
     const C* tw = reinterpret_cast<const C*>(twiddles(L, sizeof(T) == 8 ? PREC_C128 : PREC_C64));
-    const double N = (double)pl.nx * pl.ny * pl.nz;
-    const int64_t pf = tiles_in_waves(k_xcross_occ<T, L>, threads, smem, pl.pf_waves);
+      const int64_t pf = tiles_in_waves(k_xcross_occ<T, L>, threads, smem, pl.pf_waves);
     cudaError_t e = launch_pdl(k_xcross_occ<T, L>, dim3((unsigned)(rows / G)), dim3(threads), smem,
-                               s, f, tw, G, (T)(1.0 / (N * N)), pl.rev ? -pf : pf, (int)pl.rev);
+                               s, f, tw, G, (T)pl.scale2, pl.rev ? -pf : pf, (int)pl.rev);
     if (e != cudaSuccess) return cuda_status(e, "k_xcross_occ");
     return OK;
   }
@@ -548,11 +547,10 @@ int launch_xcross(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream
     attr[dev & 63] = true;
   }
   const C* tw = reinterpret_cast<const C*>(twiddles(L, sizeof(T) == 8 ? PREC_C128 : PREC_C64));
-  const double N = (double)pl.nx * pl.ny * pl.nz;
   const int blocks = (int)(rows / G);
   const int64_t pf = tiles_in_waves(k_xcross<T, L>, threads, smem, pl.pf_waves);
   cudaError_t e = launch_pdl(k_xcross<T, L>, dim3(blocks), dim3(threads), smem, s, f, tw, G,
-                             (T)(1.0 / (N * N)), pl.rev ? -pf : pf, (int)pl.rev);
+                             (T)pl.scale2, pl.rev ? -pf : pf, (int)pl.rev);
   if (e != cudaSuccess) return cuda_status(e, "k_xcross");
   return OK;
 }
@@ -600,9 +598,8 @@ int launch_xcross_tma(const NSPlan& pl, const FieldPtrs& f, int64_t rows, int* e
     set_error("twiddle table allocation failed");
     return ERR_ALLOC;
   }
-  const double N = (double)pl.nx * pl.ny * pl.nz;
   e = launch_pdl(k_xcross_tma<T, L>, dim3((unsigned)blocks), dim3(threads), smem, s, f, tw, G,
-                 (T)(1.0 / (N * N)), ntiles, (int)pl.rev, err, tma_stall_cycles());
+                 (T)pl.scale2, ntiles, (int)pl.rev, err, tma_stall_cycles());
   if (e != cudaSuccess) return cuda_status(e, "k_xcross_tma");
   return OK;
 }
@@ -744,9 +741,8 @@ int launch_xcross_r2c(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaSt
     set_error("twiddle table allocation failed");
     return ERR_ALLOC;
   }
-  const double N = (double)pl.nx_phys * pl.ny * pl.nz;
   cudaError_t e = launch_pdl(k_xcross_r2c<T, M>, dim3((unsigned)(rows / G)), dim3(threads), smem,
-                             s, f, twN, twM, G, (T)(1.0 / (N * N)), (int)pl.rev);
+                             s, f, twN, twM, G, (T)pl.scale2, (int)pl.rev);
   if (e != cudaSuccess) return cuda_status(e, "k_xcross_r2c");
   return OK;
 }

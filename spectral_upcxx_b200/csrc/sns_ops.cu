@@ -115,6 +115,40 @@ __global__ void k_vlaplacian(const cx_t<T>* __restrict__ v0, const cx_t<T>* __re
   }
 }
 
+struct BootstrapArgs {
+  const void* V0[3];
+  const void* c0[3];
+  void* V1[3];
+};
+
+// The eager sequence of ns.cpp:132-137 (about sixty field passes as single
+// operators) in one: six fields read, three written.  The divisor -|k|^2 is
+// applied in FP64 as Scalar::laplacian_inverse applies it.
+template <typename T>
+__global__ void k_bootstrap(const BootstrapArgs a, Dims d, T nu, T dt) {
+  using C = cx_t<T>;
+  const uint32_t n = (uint32_t)d.n();
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Idx p = decompose(i, d.nx, d.ny);
+    const T k[3] = {(T)freq_i(p.x, d.nx), (T)freq_i(p.y, d.ny), (T)freq_i(p.z, d.nz)};
+    const T k2 = k2_of<T>(p, d);
+    C v[3], t[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      v[q] = reinterpret_cast<const C*>(a.V0[q])[i];
+      t[q] = cadd(reinterpret_cast<const C*>(a.c0[q])[i], cscale(nu, cscale(-k2, v[q])));
+    }
+    C g = cadd(cadd(ikmul(k[0], t[0]), ikmul(k[1], t[1])), ikmul(k[2], t[2]));
+    if (k2 != (T)0) {
+      const double den = -(double)k2;
+      g = mk((T)((double)g.x / den), (T)((double)g.y / den));
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      reinterpret_cast<C*>(a.V1[q])[i] = cadd(v[q], cscale(dt, csub(t[q], ikmul(k[q], g))));
+  }
+}
+
 template <typename T>
 __global__ void k_zero_high_modes(cx_t<T>* f, Dims d) {
   // the three Nyquist planes (src/Scalar.cpp:336-370)
@@ -311,6 +345,23 @@ int op_vlaplacian(const void* const in[3], void* const out[3], Dims d, int prec,
         cp<float>(in[0]), cp<float>(in[1]), cp<float>(in[2]), mp<float>(out[0]),
         mp<float>(out[1]), mp<float>(out[2]), d);
   SNS_CHECK_LAUNCH("k_vlaplacian");
+  return OK;
+}
+
+int op_bootstrap(const void* const V0[3], const void* const c0[3], void* const V1[3], Dims d,
+                 double nu, double dt, int prec, cudaStream_t s) {
+  if (!dims_ok(d)) return ERR_ARG;
+  BootstrapArgs a{};
+  for (int q = 0; q < 3; q++) {
+    a.V0[q] = V0[q];
+    a.c0[q] = c0[q];
+    a.V1[q] = V1[q];
+  }
+  if (prec == PREC_C128)
+    k_bootstrap<double><<<grid_for(d.n()), kThreads, 0, s>>>(a, d, nu, dt);
+  else
+    k_bootstrap<float><<<grid_for(d.n()), kThreads, 0, s>>>(a, d, (float)nu, (float)dt);
+  SNS_CHECK_LAUNCH("k_bootstrap");
   return OK;
 }
 

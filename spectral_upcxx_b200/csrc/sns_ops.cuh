@@ -19,6 +19,10 @@ int op_divergence(const void* const in[3], void* out, Dims d, int prec, cudaStre
 int op_vlaplacian(const void* const in[3], void* const out[3], Dims d, int prec,
                   cudaStream_t s);
 int op_zero_high_modes(void* f, Dims d, int prec, cudaStream_t s);
+// V1 = V0 + dt (t - grad ilap(div t)) with t = c0 + nu laplacian(V0), the
+// Forward-Euler first step of ns.cpp:132-153 on Fourier fields.
+int op_bootstrap(const void* const V0[3], const void* const c0[3], void* const V1[3], Dims d,
+                 double nu, double dt, int prec, cudaStream_t s);
 // c = u x w, complex point-wise (src/Vector.cpp:79-85)
 int op_cross_pointwise(const void* const u[3], const void* const w[3], void* const c[3],
                        int64_t n, int prec, cudaStream_t s);

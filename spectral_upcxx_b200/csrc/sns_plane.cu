@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(PlaneShape<T, NX, NY>::FI * PlaneShape<T, NX, 
 }
 
 template <typename T, int NX, int NY, bool REAL>
-int launch_plane(const FieldPtrs& f, int nz, cudaStream_t s) {
+int launch_plane(const FieldPtrs& f, int nz, double scale2, cudaStream_t s) {
   using C = cx_t<T>;
   constexpr int prec = sizeof(T) == 8 ? PREC_C128 : PREC_C64;
   static bool attr[64] = {false};
@@ -152,18 +152,17 @@ int launch_plane(const FieldPtrs& f, int nz, cudaStream_t s) {
     set_error("twiddle table allocation failed");
     return ERR_ALLOC;
   }
-  const double N = (double)NX * (REAL ? 2 : 1) * NY * nz;
   cudaError_t e = launch_pdl(k_plane_cross<T, NX, NY, REAL>, dim3(nz),
                              dim3(PlaneShape<T, NX, NY>::FI * PlaneShape<T, NX, NY>::P),
-                             PlaneShape<T, NX, NY>::smem, s, f, twx, twy, twN, (T)(1.0 / (N * N)));
+                             PlaneShape<T, NX, NY>::smem, s, f, twx, twy, twN, (T)scale2);
   if (e != cudaSuccess) return cuda_status(e, "k_plane_cross");
   return OK;
 }
 
 template <typename T, int NX, int NY>
-int plane_as(const FieldPtrs& f, int nz, bool real, cudaStream_t s) {
+int plane_as(const FieldPtrs& f, int nz, bool real, double scale2, cudaStream_t s) {
   if constexpr (NX * NY * sizeof(cx_t<T>) <= 4096 * 8) {
-    return real ? launch_plane<T, NX, NY, true>(f, nz, s) : launch_plane<T, NX, NY, false>(f, nz, s);
+    return real ? launch_plane<T, NX, NY, true>(f, nz, scale2, s) : launch_plane<T, NX, NY, false>(f, nz, scale2, s);
   } else {
     set_error("plane pass: the plane does not fit a CTA");
     return ERR_UNSUPPORTED;
@@ -171,24 +170,24 @@ int plane_as(const FieldPtrs& f, int nz, bool real, cudaStream_t s) {
 }
 
 template <typename T, int NX>
-int plane_y(const FieldPtrs& f, int ny, int nz, bool real, cudaStream_t s) {
+int plane_y(const FieldPtrs& f, int ny, int nz, bool real, double scale2, cudaStream_t s) {
   switch (ny) {
-    case 16: return plane_as<T, NX, 16>(f, nz, real, s);
-    case 32: return plane_as<T, NX, 32>(f, nz, real, s);
-    case 64: return plane_as<T, NX, 64>(f, nz, real, s);
-    case 128: return plane_as<T, NX, 128>(f, nz, real, s);
-    default: return plane_as<T, NX, 256>(f, nz, real, s);
+    case 16: return plane_as<T, NX, 16>(f, nz, real, scale2, s);
+    case 32: return plane_as<T, NX, 32>(f, nz, real, scale2, s);
+    case 64: return plane_as<T, NX, 64>(f, nz, real, scale2, s);
+    case 128: return plane_as<T, NX, 128>(f, nz, real, scale2, s);
+    default: return plane_as<T, NX, 256>(f, nz, real, scale2, s);
   }
 }
 
 template <typename T>
-int plane_x(const FieldPtrs& f, int nx, int ny, int nz, bool real, cudaStream_t s) {
+int plane_x(const FieldPtrs& f, int nx, int ny, int nz, bool real, double scale2, cudaStream_t s) {
   switch (nx) {
-    case 16: return plane_y<T, 16>(f, ny, nz, real, s);
-    case 32: return plane_y<T, 32>(f, ny, nz, real, s);
-    case 64: return plane_y<T, 64>(f, ny, nz, real, s);
-    case 128: return plane_y<T, 128>(f, ny, nz, real, s);
-    default: return plane_y<T, 256>(f, ny, nz, real, s);
+    case 16: return plane_y<T, 16>(f, ny, nz, real, scale2, s);
+    case 32: return plane_y<T, 32>(f, ny, nz, real, scale2, s);
+    case 64: return plane_y<T, 64>(f, ny, nz, real, scale2, s);
+    case 128: return plane_y<T, 128>(f, ny, nz, real, scale2, s);
+    default: return plane_y<T, 256>(f, ny, nz, real, scale2, s);
   }
 }
 
@@ -200,16 +199,18 @@ bool plane_supported(int nx, int ny, int prec) {
          (size_t)nx * ny * esz <= 4096 * 8;
 }
 
-int plane_run(void* const U[6], int nx, int ny, int nz, int prec, bool real, cudaStream_t s) {
+int plane_run(void* const in[6], void* const out[3], int nx, int ny, int nz, int prec, bool real,
+              double scale2, cudaStream_t s) {
   if (!plane_supported(nx, ny, prec)) {
     set_error("plane pass: the plane does not fit a CTA");
     return ERR_UNSUPPORTED;
   }
   FieldPtrs f{};
   f.n = 6;
-  for (int i = 0; i < 6; i++) f.in[i] = f.out[i] = U[i];
-  return prec == PREC_C128 ? plane_x<double>(f, nx, ny, nz, real, s)
-                           : plane_x<float>(f, nx, ny, nz, real, s);
+  for (int i = 0; i < 6; i++) f.in[i] = in[i];
+  for (int i = 0; i < 3; i++) f.out[i] = out[i];
+  return prec == PREC_C128 ? plane_x<double>(f, nx, ny, nz, real, scale2, s)
+                           : plane_x<float>(f, nx, ny, nz, real, scale2, s);
 }
 
 }  // namespace sns

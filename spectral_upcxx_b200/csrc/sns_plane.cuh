@@ -9,8 +9,10 @@ namespace sns {
 
 // Whether a CTA can hold the six fields' plane of stored rows of nx values.
 bool plane_supported(int nx, int ny, int prec);
-// The xy phase of nz planes in place on U[0..5]: U[0..2] = y- and x-transformed
-// cross product (U[3..5] are left as they were).  real: half-spectrum rows.
-int plane_run(void* const U[6], int nx, int ny, int nz, int prec, bool real, cudaStream_t s);
+// The xy phase of nz planes: out[0..2] = scale2 (in[0..2] x in[3..5]), both
+// y- and x-inverse-transformed before and y- and x-forward-transformed after
+// (out may be in[0..2]).  real: half-spectrum rows.
+int plane_run(void* const in[6], void* const out[3], int nx, int ny, int nz, int prec, bool real,
+              double scale2, cudaStream_t s);
 
 }  // namespace sns
