@@ -242,7 +242,12 @@ static void choose_tile(LineGeo& g, int64_t adjacent, int64_t groups, int prec, 
          (size_t)(W * 2) * tile_stride(g.L, W * 2, (int)esz) * esz <= smem_cap)
     W *= 2;
   int G = 1;
-  const int tcap = tmax > 0 ? tmax : 256;  // threads per CTA up to which groups are added
+  // threads per CTA up to which groups are added.  Small CTAs drift apart, so
+  // one's loads run under another's transforms: B200, forward + inverse at
+  // 64 / 128 / 256 threads: 256^3 complex128 537 / 539 / 616 us, 128^3
+  // complex128 of 6 fields 433 / 435 / 448 us, 64^3 complex64 of 6 fields 49 /
+  // 53 / 53 us.
+  const int tcap = tmax > 0 ? tmax : 64;
   while (W * G * 2 * TPL <= tcap && W * G * 2 * TPL <= max_threads(prec) &&
          groups % (G * 2) == 0 &&
          (size_t)(W * G * 2) * tile_stride(g.L, W, (int)esz) * esz <= smem_cap / 2)

@@ -300,13 +300,11 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   pl.lineW = lineW > 0 ? lineW : 0;
   pl.lineT = 0;
   pl.lineOrd = 0;
-  // y passes of fields beyond L2: one line group per CTA of up to 128 threads
-  // (or one run of W lines), in complex64 over TMA-staged tiles.  B200, 256^3,
-  // both passes: complex64 0.427 ms against 0.491 (direct loads, 256 threads);
-  // complex128 0.820 against 0.908 (256 threads; staged 0.87).
-  if (big && lineW <= 0 && !getenv("SNS_LINE_W")) pl.lineT = 128;
   {
-    // SNS_Y_TMA = 0 (direct loads), 1 or 2 stages
+    // The y passes of fields beyond L2 over TMA-staged tiles in complex64
+    // (SNS_Y_TMA = 0: direct loads, 1 or 2 stages).  B200, 256^3, both passes:
+    // complex64 0.427 ms against 0.491 with direct loads; complex128 0.87
+    // against 0.82.
     const char* e = getenv("SNS_Y_TMA");
     const int v = e ? atoi(e) : big && prec == PREC_C64 ? 1 : 0;
     pl.y_tma = 0;
