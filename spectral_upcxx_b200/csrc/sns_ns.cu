@@ -66,8 +66,8 @@ namespace {
 // K3 of the plan: complex rows, or half-spectrum rows of a real-field run
 int xpass(const NSPlan& pl, const FieldPtrs& f, int64_t rows, int* err, cudaStream_t s) {
   if (pl.real)
-    return pl.prec == PREC_C128 ? ns_xcross_r2c<double>(pl, f, rows, s)
-                                : ns_xcross_r2c<float>(pl, f, rows, s);
+    return pl.prec == PREC_C128 ? ns_xcross_real<double>(pl, f, rows, s)
+                                : ns_xcross_real<float>(pl, f, rows, s);
   return pl.prec == PREC_C128 ? ns_xcross<double>(pl, f, rows, err, s)
                               : ns_xcross<float>(pl, f, rows, err, s);
 }
@@ -154,8 +154,9 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   // fields beyond L2: the step streams from HBM
   const bool big = !ns_fits_l2(pl);
   {
-    const int TPL = nx / elems(nx);
-    const int G = x_tile_rows(nx, (int64_t)ny * nz, prec);
+    // (a real-field run: pairs of rows, as lines of the physical nx)
+    const int TPL = pl.nx_phys / elems(pl.nx_phys);
+    const int G = x_tile_rows(pl.nx_phys, (int64_t)ny * nz / (real ? 2 : 1), prec);
     pl.scale2 = 1.0 / (((double)pl.nx_phys * ny * nz) * ((double)pl.nx_phys * ny * nz));
     if (6 * G * TPL > max_threads(prec)) {
       set_error("fused NS step: nx too large for the x-pass tile");
@@ -588,11 +589,11 @@ bool k1_ok(const NSPlan& p, int W, int G, bool reload) {
          (size_t)(reload ? 3 : 6) * W * G * tile_stride(p.nz, W, (int)esz) * esz <= kTuneSmemCap;
 }
 bool xg_ok(const NSPlan& p, int G) {
-  const int TPL = p.nx / elems(p.nx);
+  const int TPL = p.nx_phys / elems(p.nx_phys);
   const size_t esz = p.prec == PREC_C128 ? 16 : 8;
-  const int cap = p.real ? 384 : max_threads(p.prec);  // k_xcross_r2c launch bound
-  return ((int64_t)p.ny * p.nz) % G == 0 && 6 * G * TPL <= cap &&
-         (size_t)6 * G * xrow_stride(p.nx, (int)esz) * esz <= kTuneSmemCap;
+  const int cap = p.real ? 384 : max_threads(p.prec);  // k_xcross_real launch bound
+  return ((int64_t)p.ny * p.nz) % (p.real ? 2 * G : G) == 0 && 6 * G * TPL <= cap &&
+         (size_t)6 * G * xrow_stride(p.nx_phys, (int)esz) * esz <= kTuneSmemCap;
 }
 bool zw_ok(const NSPlan& p, int W, int max_blocks, bool halves = false) {
   const int TPL = p.nz / elems(p.nz);

@@ -92,7 +92,7 @@ inline bool z_tma_ok(const NSPlan& p, int W) {
 template <typename T>
 int ns_xcross(const NSPlan& pl, const FieldPtrs& f, int64_t rows, int* err, cudaStream_t s);
 template <typename T>
-int ns_xcross_r2c(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream_t s);
+int ns_xcross_real(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream_t s);
 template <typename T>
 int ns_zcurl(const NSPlan& pl, const FieldPtrs& f, int* err, cudaStream_t s);
 template <typename T, bool SGS>
@@ -203,79 +203,16 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 }
 
 // ---------------------------------------------------------------------------
-// K3 of a real-field run (r2c_rows_pre, r2c_rows_post in sns_tiles.cuh).  twN:
-// the 2M-point table exp(-2 pi i m / 2M); twM: the M-point table.  No line
-// values stay in registers across the pre- and post-processing; FP32 fits two
-// CTAs per SM.
-template <typename T, int M>
+// K3 of a real-field run: G pairs of rows of L / 2 half-spectrum values.
+template <typename T, int L>
 __global__ void __launch_bounds__(384, sizeof(T) == 4 ? 2 : 1)
-    k_xcross_r2c(FieldPtrs f, const cx_t<T>* __restrict__ twN, const cx_t<T>* __restrict__ twM,
-                 int G, T scale2, int rev) {
-  using C = cx_t<T>;
-  using P = LinePlan<M>;
-  constexpr int E = P::E, TPL = P::TPL, RS = xrow_stride(M, (int)sizeof(C));
-  static_assert(TPL <= 32, "a line's threads share a warp");
+    k_xcross_real(FieldPtrs f, const cx_t<T>* __restrict__ tw, int G, T scale2, int rev) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_trigger();
   pdl_wait();
-  C* sm = reinterpret_cast<C*>(smem_raw);
-  const int64_t row0 = tile_order((int64_t)blockIdx.x, (int64_t)gridDim.x, rev) * G;
-  const int per = G * M;
-  const int j = threadIdx.x % TPL, line = threadIdx.x / TPL;
-  const int fld = line / G, gl = line - fld * G;
-  C* row = sm + line * RS;
-  C v[E];
-  {
-    const C* __restrict__ src = reinterpret_cast<const C*>(select_ptr(f.in, fld));
-    const int64_t i0 = (row0 + gl) * M + j;
-#pragma unroll
-    for (int e = 0; e < E; e++) v[e] = src[i0 + TPL * e];
-  }
-#pragma unroll
-  for (int e = 0; e < E; e++) row[pad_pos(j + TPL * e)] = v[e];
-  line_sync<TPL>();
-  r2c_rows_pre<M>(row, j, twN);
-  line_sync<TPL>();
-#pragma unroll
-  for (int e = 0; e < E; e++) v[e] = row[pad_pos(j + TPL * e)];
-  line_sync<TPL>();
-  line_fft<M>(v, row, j, twM, (T)1);
-#pragma unroll
-  for (int e = 0; e < E; e++) row[pad_pos(j + TPL * e)] = v[e];
-  __syncthreads();
-
-  // c = (u/N) x (omega/N) on the real samples (.x and .y of each slot)
-  for (int q = threadIdx.x; q < per; q += blockDim.x) {
-    const int g = q / M, p = q & (M - 1);
-    C u[3], w[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      u[d] = sm[(d * G + g) * RS + pad_pos(p)];
-      w[d] = sm[((3 + d) * G + g) * RS + pad_pos(p)];
-    }
-    C c[3];
-    cross_point<true>(u, w, scale2, c);
-#pragma unroll
-    for (int d = 0; d < 3; d++) sm[(d * G + g) * RS + pad_pos(p)] = c[d];
-  }
-  __syncthreads();
-
-  // forward: warps holding only omega rows skip it (as in k_xcross)
-  constexpr int kLinesPerWarp = 32 / TPL;
-  const bool skip = (G % kLinesPerWarp == 0) && fld >= 3;
-  if (!skip) {
-#pragma unroll
-    for (int e = 0; e < E; e++) v[e] = row[pad_pos(j + TPL * e)];
-    line_sync<TPL>();
-    line_fft<M>(v, row, j, twM, (T)-1);
-#pragma unroll
-    for (int e = 0; e < E; e++) row[pad_pos(j + TPL * e)] = v[e];
-    line_sync<TPL>();
-  }
-  if (fld < 3) {
-    C* __restrict__ dst = reinterpret_cast<C*>(select_ptr(f.out, fld)) + (row0 + gl) * M;
-    r2c_rows_post<M>(row, j, twN, [&](int k, C c) { dst[k] = c; });
-  }
+  xcross_real_tile<T, L>(ParamFields{f}, tw, G, scale2,
+                         tile_order((int64_t)blockIdx.x, (int64_t)gridDim.x, rev),
+                         (int)blockDim.x, reinterpret_cast<cx_t<T>*>(smem_raw));
 }
 
 // ---------------------------------------------------------------------------
@@ -719,31 +656,29 @@ int launch_zcurl(const NSPlan& pl, const FieldPtrs& f, int* err, cudaStream_t s)
                       : launch_zcurl_as<T, L, false>(pl, f, s);
 }
 
-template <typename T, int M>
-int launch_xcross_r2c(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream_t s) {
+template <typename T, int L>
+int launch_xcross_real(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream_t s) {
   using C = cx_t<T>;
-  constexpr int TPL = LinePlan<M>::TPL;
+  constexpr int TPL = LinePlan<L>::TPL;
   const int G = pl.xG;
   const int threads = 6 * G * TPL;
-  const size_t smem = (size_t)6 * G * xrow_stride(M, (int)sizeof(C)) * sizeof(C);
+  const size_t smem = (size_t)6 * G * xrow_stride(L, (int)sizeof(C)) * sizeof(C);
   static bool attr[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr[dev & 63]) {
-    cudaError_t e = allow_max_dynamic_smem(k_xcross_r2c<T, M>);
-    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(k_xcross_r2c)");
+    cudaError_t e = allow_max_dynamic_smem(k_xcross_real<T, L>);
+    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(k_xcross_real)");
     attr[dev & 63] = true;
   }
-  const int prec = sizeof(T) == 8 ? PREC_C128 : PREC_C64;
-  const C* twN = reinterpret_cast<const C*>(twiddles(2 * M, prec));
-  const C* twM = reinterpret_cast<const C*>(twiddles(M, prec));
-  if (!twN || !twM) {
+  const C* tw = reinterpret_cast<const C*>(twiddles(L, sizeof(T) == 8 ? PREC_C128 : PREC_C64));
+  if (!tw) {
     set_error("twiddle table allocation failed");
     return ERR_ALLOC;
   }
-  cudaError_t e = launch_pdl(k_xcross_r2c<T, M>, dim3((unsigned)(rows / G)), dim3(threads), smem,
-                             s, f, twN, twM, G, (T)pl.scale2, (int)pl.rev);
-  if (e != cudaSuccess) return cuda_status(e, "k_xcross_r2c");
+  cudaError_t e = launch_pdl(k_xcross_real<T, L>, dim3((unsigned)(rows / (2 * G))), dim3(threads),
+                             smem, s, f, tw, G, (T)pl.scale2, (int)pl.rev);
+  if (e != cudaSuccess) return cuda_status(e, "k_xcross_real");
   return OK;
 }
 
@@ -852,14 +787,14 @@ int launch_update_tma(const NSPlan& pl, const UpdateArgs& a, int* err, cudaStrea
 }  // namespace
 
 template <typename T>
-int ns_xcross_r2c(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream_t s) {
-  switch (pl.nx) {
-    case 16: return launch_xcross_r2c<T, 16>(pl, f, rows, s);
-    case 32: return launch_xcross_r2c<T, 32>(pl, f, rows, s);
-    case 64: return launch_xcross_r2c<T, 64>(pl, f, rows, s);
-    case 128: return launch_xcross_r2c<T, 128>(pl, f, rows, s);
-    case 256: return launch_xcross_r2c<T, 256>(pl, f, rows, s);
-    case 512: return launch_xcross_r2c<T, 512>(pl, f, rows, s);
+int ns_xcross_real(const NSPlan& pl, const FieldPtrs& f, int64_t rows, cudaStream_t s) {
+  switch (pl.nx_phys) {
+    case 32: return launch_xcross_real<T, 32>(pl, f, rows, s);
+    case 64: return launch_xcross_real<T, 64>(pl, f, rows, s);
+    case 128: return launch_xcross_real<T, 128>(pl, f, rows, s);
+    case 256: return launch_xcross_real<T, 256>(pl, f, rows, s);
+    case 512: return launch_xcross_real<T, 512>(pl, f, rows, s);
+    case 1024: return launch_xcross_real<T, 1024>(pl, f, rows, s);
     default: set_error("real-field NS step: nx must be a power of two in [32, 1024]"); return ERR_UNSUPPORTED;
   }
 }
@@ -953,7 +888,7 @@ int ns_update_carry(const NSPlan& pl, const UpdateArgs& a, cudaStream_t s) {
 // Every pass at precision T (once per source file that defines SNS_NS_PASSES).
 #define SNS_NS_PASSES_OF(T)                                                                   \
   template int ns_xcross<T>(const NSPlan&, const FieldPtrs&, int64_t, int*, cudaStream_t);    \
-  template int ns_xcross_r2c<T>(const NSPlan&, const FieldPtrs&, int64_t, cudaStream_t);      \
+  template int ns_xcross_real<T>(const NSPlan&, const FieldPtrs&, int64_t, cudaStream_t);      \
   template int ns_zcurl<T>(const NSPlan&, const FieldPtrs&, int*, cudaStream_t);              \
   template int ns_update_as<T, true>(const NSPlan&, const UpdateArgs&, int*, cudaStream_t);   \
   template int ns_update_as<T, false>(const NSPlan&, const UpdateArgs&, int*, cudaStream_t);  \

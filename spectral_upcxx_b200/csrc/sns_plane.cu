@@ -33,21 +33,23 @@ struct PlaneShape {
   static constexpr int RS = xrow_stride(NX, (int)sizeof(cx_t<T>), E);
   static constexpr int FS = NY * RS;                 // slots per field
   static constexpr size_t smem = (size_t)6 * FS * sizeof(cx_t<T>);
-  using X = LinePlan<NX, RADIX16_FIRST, E>;
   using Y = LinePlan<NY, RADIX16_FIRST, E>;
 };
 
-// REAL: rows of NX half-spectrum values of a real line of 2 NX points; twN is
-// then the table of 2 NX.
+// REAL: rows of NX half-spectrum values of real lines of 2 NX points; the x
+// lines are pairs of rows (real_pair_load), in the pair's slots.  twx: the table
+// of the x lines' length.
 template <typename T, int NX, int NY, bool REAL>
 __global__ void __launch_bounds__(PlaneShape<T, NX, NY>::FI * PlaneShape<T, NX, NY>::P)
     k_plane_cross(const FieldPtrs f, const cx_t<T>* __restrict__ twx,
-                  const cx_t<T>* __restrict__ twy, const cx_t<T>* __restrict__ twN, T scale2) {
+                  const cx_t<T>* __restrict__ twy, T scale2) {
   using C = cx_t<T>;
   using SH = PlaneShape<T, NX, NY>;
   constexpr int E = SH::E, P = SH::P, FI = SH::FI, RS = SH::RS, FS = SH::FS;
-  constexpr int TX = SH::X::TPL, TY = SH::Y::TPL;
-  static_assert(SH::X::E == E && SH::Y::E == E && TX <= 32, "plane tile");
+  constexpr int LX = REAL ? 2 * NX : NX;       // points of an x line
+  constexpr int RX = REAL ? 2 * RS : RS;       // slots of an x line
+  constexpr int TX = LX / E, TY = SH::Y::TPL;
+  static_assert(LinePlan<LX, RADIX16_FIRST, E>::E == E && SH::Y::E == E && TX <= 32, "plane tile");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* sm = reinterpret_cast<C*>(smem_raw);
   const int fi = threadIdx.x / P, t = threadIdx.x % P;
@@ -77,21 +79,21 @@ __global__ void __launch_bounds__(PlaneShape<T, NX, NY>::FI * PlaneShape<T, NX, 
   // x-inverse in place
 #pragma unroll 1
   for (int f0 = 0; f0 < 6; f0 += FI) {
-    C* row = sm + (f0 + fi) * FS + ry * RS;
-    if constexpr (REAL) {
-      r2c_rows_pre<NX, TX>(row, rj, twN);
-      line_sync<TX>();
-    }
+    C* row = sm + (f0 + fi) * FS + ry * RX;
+    if constexpr (REAL)
+      real_pair_load<LX>(
+          v, rj, [&](int k) { return row[pad_pos(k)]; }, [&](int k) { return row[RS + pad_pos(k)]; });
+    else
 #pragma unroll
-    for (int e = 0; e < E; e++) v[e] = row[pad_pos(rj + TX * e)];
+      for (int e = 0; e < E; e++) v[e] = row[pad_pos(rj + TX * e)];
     line_sync<TX>();
-    line_fft<NX, false, RADIX16_FIRST, E>(v, row, rj, twx, (T)1);
+    line_fft<LX, false, RADIX16_FIRST, E>(v, row, rj, twx, (T)1);
 #pragma unroll
     for (int e = 0; e < E; e++) row[pad_pos(rj + TX * e)] = v[e];
   }
   __syncthreads();
   for (int q = threadIdx.x; q < NX * NY; q += FI * P) {
-    C* at = sm + (q / NX) * RS + pad_pos(q % NX);
+    C* at = sm + (q / LX) * RX + pad_pos(q % LX);
     C u[3], w[3], c[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -107,16 +109,21 @@ __global__ void __launch_bounds__(PlaneShape<T, NX, NY>::FI * PlaneShape<T, NX, 
   C* fld = sm + fi * FS;
   // whole warps of the fields 3..5 skip the x lines
   if (fi < 3 || P % 32 != 0) {
-    C* row = fld + ry * RS;
+    C* row = fld + ry * RX;
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = row[pad_pos(rj + TX * e)];
     line_sync<TX>();
-    line_fft<NX, false, RADIX16_FIRST, E>(v, row, rj, twx, (T)-1);
-#pragma unroll
-    for (int e = 0; e < E; e++) row[pad_pos(rj + TX * e)] = v[e];
+    line_fft<LX, false, RADIX16_FIRST, E>(v, row, rj, twx, (T)-1);
     if constexpr (REAL) {
+      C zn[E / 2];
+      real_pair_mirror<LX>(v, zn, row, rj, [] { line_sync<TX>(); });
       line_sync<TX>();
-      r2c_rows_post<NX, TX>(row, rj, twN, [&](int k, C c) { row[pad_pos(k)] = c; });
+#pragma unroll
+      for (int e = 0; e < E / 2; e++)
+        real_pair_split(v[e], zn[e], &row[pad_pos(rj + TX * e)], &row[RS + pad_pos(rj + TX * e)]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; e++) row[pad_pos(rj + TX * e)] = v[e];
     }
   }
   __syncthreads();
@@ -145,16 +152,15 @@ int launch_plane(const FieldPtrs& f, int nz, double scale2, cudaStream_t s) {
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(k_plane_cross)");
     attr[dev & 63] = true;
   }
-  const C* twx = reinterpret_cast<const C*>(twiddles(NX, prec));
+  const C* twx = reinterpret_cast<const C*>(twiddles(REAL ? 2 * NX : NX, prec));
   const C* twy = reinterpret_cast<const C*>(twiddles(NY, prec));
-  const C* twN = REAL ? reinterpret_cast<const C*>(twiddles(2 * NX, prec)) : twx;
-  if (!twx || !twy || !twN) {
+  if (!twx || !twy) {
     set_error("twiddle table allocation failed");
     return ERR_ALLOC;
   }
   cudaError_t e = launch_pdl(k_plane_cross<T, NX, NY, REAL>, dim3(nz),
                              dim3(PlaneShape<T, NX, NY>::FI * PlaneShape<T, NX, NY>::P),
-                             PlaneShape<T, NX, NY>::smem, s, f, twx, twy, twN, (T)scale2);
+                             PlaneShape<T, NX, NY>::smem, s, f, twx, twy, (T)scale2);
   if (e != cudaSuccess) return cuda_status(e, "k_plane_cross");
   return OK;
 }
