@@ -48,6 +48,11 @@ template <typename C>
 __device__ __forceinline__ C cmul(C a, C b) {
   return mk(fma_rn(a.x, b.x, -mul_rn(a.y, b.y)), fma_rn(a.x, b.y, mul_rn(a.y, b.x)));
 }
+// a + i sg d (sg = +-1: the product is exact)
+template <typename C, typename T>
+__device__ __forceinline__ C caddi(C a, C d, T sg) {
+  return mk(a.x - sg * d.y, a.y + sg * d.x);
+}
 // i (ka a - kb b): one component of the curl i k x v.
 template <typename C, typename T>
 __device__ __forceinline__ C curl_part(T ka, C a, T kb, C b) {

@@ -117,11 +117,10 @@ __device__ __forceinline__ void dft(C* a, T sg) {
   } else if constexpr (R == 4) {
     C t0 = cadd(a[0], a[2]), t1 = csub(a[0], a[2]);
     C t2 = cadd(a[1], a[3]), d = csub(a[1], a[3]);
-    C t3 = mk(-sg * d.y, sg * d.x);  // d * (sg i)
     a[0] = cadd(t0, t2);
     a[2] = csub(t0, t2);
-    a[1] = cadd(t1, t3);
-    a[3] = csub(t1, t3);
+    a[1] = caddi(t1, d, sg);
+    a[3] = caddi(t1, d, -sg);
   } else {
     // radix-2 decimation in time: R = 2 * (R/2)
     constexpr int H = R / 2;
@@ -135,18 +134,18 @@ __device__ __forceinline__ void dft(C* a, T sg) {
     dft<H>(o, sg);
 #pragma unroll
     for (int k = 0; k < H; k++) {
-      C t;
-      if (k == 0) {
-        t = o[0];
-      } else if (2 * k == H) {
-        t = mk(-sg * o[k].y, sg * o[k].x);  // W_R^{R/4} = sg i
+      if (2 * k == H) {  // W_R^{R/4} = sg i
+        a[k] = caddi(e[k], o[k], sg);
+        a[k + H] = caddi(e[k], o[k], -sg);
       } else {
-        constexpr int step = 16 / R;
-        const T c = (T)tw16_c(k * step), s = sg * (T)tw16_s(k * step);
-        t = cmul(o[k], mk(c, s));
+        C t = o[k];
+        if (k > 0) {
+          constexpr int step = 16 / R;
+          t = cmul(t, mk((T)tw16_c(k * step), sg * (T)tw16_s(k * step)));
+        }
+        a[k] = cadd(e[k], t);
+        a[k + H] = csub(e[k], t);
       }
-      a[k] = cadd(e[k], t);
-      a[k + H] = csub(e[k], t);
     }
   }
 }

@@ -486,9 +486,10 @@ __device__ __forceinline__ void cross_point(const C (&u)[3], const C (&w)[3], T 
   for (int d = 0; d < 3; d++) {
     const C &ua = u[(d + 1) % 3], &ub = u[(d + 2) % 3];
     const C &wa = w[(d + 1) % 3], &wb = w[(d + 2) % 3];
-    const C p = REAL ? mk(fma_rn(ua.x, wb.x, -mul_rn(ub.x, wa.x)),
-                          fma_rn(ua.y, wb.y, -mul_rn(ub.y, wa.y)))
-                     : csub(cmul(ua, wb), cmul(ub, wa));
+    const C p =
+        REAL ? mk(fma_rn(ua.x, wb.x, -mul_rn(ub.x, wa.x)), fma_rn(ua.y, wb.y, -mul_rn(ub.y, wa.y)))
+             : mk(fma_rn(ua.x, wb.x, fma_rn(-ua.y, wb.y, fma_rn(-ub.x, wa.x, mul_rn(ub.y, wa.y)))),
+                  fma_rn(ua.x, wb.y, fma_rn(ua.y, wb.x, fma_rn(-ub.x, wa.y, -mul_rn(ub.y, wa.x)))));
     c[d] = mk(mul_rn(scale2, p.x), mul_rn(scale2, p.y));
   }
 }
