@@ -285,6 +285,7 @@ using namespace sns;
 // idles for about 2 us, which a step of such a box (10 to 100 us) feels.  B200,
 // complex64: 32^3 14.8 -> 12.4 us a step, 64^3 31.2 -> 29.7 us.
 constexpr int kBatchSteps = 8;
+static_assert(kBatchSteps % 2 == 0, "a batch leaves the history where it was");
 
 // ---- stepper object ----------------------------------------------------------
 struct sns_ns {
@@ -302,6 +303,8 @@ struct sns_ns {
   // U holds K1's output for the current V (left there by a carrying K5); any
   // call that writes V or U other than a plain step clears it
   bool carried = false;
+  // where the history cross0 is (HIST_*)
+  int hist = HIST_FOURIER;
   // eddy-viscosity closure (none by default) and its six extra work fields
   Closure cl;
   void* U2[6] = {};
@@ -314,24 +317,35 @@ struct sns_ns {
   bool use_graph = true;
   bool eager_done = false;
   cudaStream_t cap = nullptr;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  // [history in C0, in U or Fourier]: a plain step's fields take turns
+  cudaGraph_t graph[2] = {};
+  cudaGraphExec_t exec[2] = {};
   // kBatchSteps steps in one graph, for boxes whose step is a few microseconds
-  cudaGraph_t batch_graph = nullptr;
-  cudaGraphExec_t batch = nullptr;
+  cudaGraph_t batch_graph[2] = {};
+  cudaGraphExec_t batch[2] = {};
 };
 
 namespace {
 
 void drop_graph(sns_ns* h) {
-  if (h->exec) cudaGraphExecDestroy(h->exec);
-  if (h->graph) cudaGraphDestroy(h->graph);
-  h->exec = nullptr;
-  h->graph = nullptr;
-  if (h->batch) cudaGraphExecDestroy(h->batch);
-  if (h->batch_graph) cudaGraphDestroy(h->batch_graph);
-  h->batch = nullptr;
-  h->batch_graph = nullptr;
+  for (int i = 0; i < 2; i++) {
+    if (h->exec[i]) cudaGraphExecDestroy(h->exec[i]);
+    if (h->graph[i]) cudaGraphDestroy(h->graph[i]);
+    if (h->batch[i]) cudaGraphExecDestroy(h->batch[i]);
+    if (h->batch_graph[i]) cudaGraphDestroy(h->batch_graph[i]);
+    h->exec[i] = h->batch[i] = nullptr;
+    h->graph[i] = h->batch_graph[i] = nullptr;
+  }
+}
+
+// The history into its Fourier form in C0, for what reads it there.
+int hist_to_fourier(sns_ns* h) {
+  if (h->hist == HIST_FOURIER) return OK;
+  const int rc = ns_hist_fourier(h->pl, h->hist == HIST_Z_U ? h->U : h->C0, h->C0, 3, h->s);
+  if (rc) return rc;
+  h->hist = HIST_FOURIER;
+  h->carried = false;  // U[0..2] or C0 no longer is what a carried K1 wrote
+  return OK;
 }
 
 // One step (plain or closure) queued on `s`.
@@ -342,11 +356,12 @@ int step_on(sns_ns* h, cudaStream_t s, cudaEvent_t* ev) {
       U[i] = h->U[i];
       U[6 + i] = h->U2[i];
     }
+    if (int rc = hist_to_fourier(h)) return rc;
     h->carried = false;  // the closure step uses U as work space
     return les_step_once(h->pl, h->V, h->C0, U, h->stats_part, h->nu, h->dt, h->cl, s);
   }
   return ns_step_once(h->pl, h->V, h->C0, h->U, h->stats_part, h->sync_words, h->nu, h->dt, s,
-                      ev, h->W, &h->carried);
+                      ev, h->W, &h->carried, &h->hist);
 }
 
 int capture_steps(sns_ns* h, int steps, cudaGraph_t* graph, cudaGraphExec_t* exec) {
@@ -358,8 +373,13 @@ int capture_steps(sns_ns* h, int steps, cudaGraph_t* graph, cudaGraphExec_t* exe
   if ((rc = cuda_status(cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal),
                         "sns_ns_step(capture)")))
     return rc;
+  // the captured steps have not run: where the fields are is as before
+  const int hist = h->hist;
+  const bool carried = h->carried;
   int src = OK;
   for (int t = 0; t < steps && !src; t++) src = step_on(h, h->cap, nullptr);
+  h->hist = hist;
+  h->carried = carried;
   cudaGraph_t g = nullptr;
   rc = cuda_status(cudaStreamEndCapture(h->cap, &g), "sns_ns_step(capture)");
   if (src || rc) {
@@ -781,6 +801,7 @@ int sns_ns_set_state(sns_ns* h, const void* const V1[3], const void* const cross
     if (rc) return rc;
     h->stepped = false;
     h->carried = false;
+    h->hist = HIST_FOURIER;
     return OK;
   }
   const size_t bytes = esize(h->pl.prec) * (size_t)h->pl.nx * h->pl.ny * h->pl.nz;
@@ -796,6 +817,7 @@ int sns_ns_set_state(sns_ns* h, const void* const V1[3], const void* const cross
   }
   h->stepped = false;
   h->carried = false;
+  h->hist = HIST_FOURIER;
   return OK;
 }
 
@@ -820,6 +842,7 @@ int sns_ns_bootstrap(sns_ns* h, const void* const V0[3], const void* const omega
     if (rc) return rc;
     h->stepped = false;
     h->carried = false;
+    h->hist = HIST_FOURIER;
     return OK;
   }
   const Dims d{h->pl.nx, h->pl.ny, h->pl.nz};
@@ -827,6 +850,7 @@ int sns_ns_bootstrap(sns_ns* h, const void* const V0[3], const void* const omega
   if (rc) return rc;
   h->stepped = false;
   h->carried = false;
+  h->hist = HIST_FOURIER;
   return OK;
 }
 
@@ -844,19 +868,24 @@ int sns_ns_step(sns_ns* h, int nsteps) {
       int rc = OK;
       // a captured step of a carrying plan starts from K1's output in U:
       // make it there first if the state was set since
-      if (h->pl.carry && !h->carried && h->cl.model == CLOSURE_NONE && h->use_graph &&
-          h->eager_done) {
-        if ((rc = ns_k1_once(h->pl, h->V, h->U, h->sync_words, h->s))) return rc;
+      // (a Fourier history serves the one step after it was set, launched directly)
+      const bool plain = h->cl.model == CLOSURE_NONE;
+      const bool replay = h->use_graph && h->eager_done && !(plain && h->hist == HIST_FOURIER);
+      if (replay && plain && h->pl.carry && !h->carried) {
+        if ((rc = ns_k1_once(h->pl, h->V, h->C0, h->U, h->hist, h->sync_words, h->s))) return rc;
         h->carried = true;
       }
       const bool whole = small && nsteps - t >= kBatchSteps;
-      if (h->use_graph && h->eager_done) {
-        if (whole && !h->batch)
-          rc = capture_steps(h, kBatchSteps, &h->batch_graph, &h->batch);
-        else if (!whole && !h->exec)
-          rc = capture_steps(h, 1, &h->graph, &h->exec);
+      if (replay) {
+        const int i = plain && h->hist == HIST_Z_C0 ? 0 : 1;
+        if (whole && !h->batch[i])
+          rc = capture_steps(h, kBatchSteps, &h->batch_graph[i], &h->batch[i]);
+        else if (!whole && !h->exec[i])
+          rc = capture_steps(h, 1, &h->graph[i], &h->exec[i]);
         if (rc) return rc;
-        rc = cuda_status(cudaGraphLaunch(whole ? h->batch : h->exec, h->s), "sns_ns_step(graph)");
+        rc = cuda_status(cudaGraphLaunch(whole ? h->batch[i] : h->exec[i], h->s),
+                         "sns_ns_step(graph)");
+        if (!rc && plain && !whole) h->hist = i == 0 ? HIST_Z_U : HIST_Z_C0;
         t += whole ? kBatchSteps : 1;
       } else {
         rc = step_on(h, h->s, nullptr);
@@ -885,7 +914,7 @@ int sns_ns_step(sns_ns* h, int nsteps) {
       ev = &h->events[(size_t)h->recorded * (kNSPasses + 1)];
     }
     int rc = ns_step_once(h->pl, h->V, h->C0, h->U, h->stats_part, h->sync_words, h->nu, h->dt,
-                          h->s, ev, h->W, &h->carried);
+                          h->s, ev, h->W, &h->carried, &h->hist);
     if (rc) return rc;
     if (ev) h->recorded++;
     h->stepped = true;
@@ -930,8 +959,20 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
     const Dims d{h->pl.nx_phys, h->pl.ny, h->pl.nz};
     const size_t bytes = esize(h->pl.prec) * (size_t)d.n();
     int rc = OK;
-    if (cross0 && cross0[0] && cross0[1] && cross0[2])
-      rc = convert_half(cross0, h->C0, d.nx, d.ny, d.nz, h->pl.prec, -1, h->s);
+    if (cross0 && cross0[0] && cross0[1] && cross0[2]) {
+      void* c[3] = {h->C0[0], h->C0[1], h->C0[2]};
+      const bool z = h->hist != HIST_FOURIER;
+      if (z) {
+        for (int i = 0; i < 3; i++) c[i] = nullptr;
+        for (int i = 0; i < 3 && !rc; i++) rc = pool_malloc(&c[i], bytes / 2);
+        if (!rc) rc = ns_hist_fourier(h->pl, h->hist == HIST_Z_U ? h->U : h->C0, c, 3, h->s);
+      }
+      if (!rc) rc = convert_half(cross0, c, d.nx, d.ny, d.nz, h->pl.prec, -1, h->s);
+      if (z) {
+        cudaStreamSynchronize(h->s);
+        for (void* p : c) pool_free(p);
+      }
+    }
     if (rc || (!omega1 && !(V1 && V1[0] && V1[1] && V1[2]))) return rc;
     void* t[3] = {};
     const bool own = !(V1 && V1[0] && V1[1] && V1[2]);
@@ -958,16 +999,30 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
   const Dims d{h->pl.nx, h->pl.ny, h->pl.nz};
   const size_t bytes = esize(h->pl.prec) * (size_t)d.n();
   int rc;
+  // a destination that only a byte copy can write
+  for (int i = 0; i < 3 && cross0; i++)
+    if (reinterpret_cast<uintptr_t>(cross0[i]) % esize(h->pl.prec))
+      if ((rc = hist_to_fourier(h))) return rc;
   for (int i = 0; i < 3; i++) {
     if (V1 && V1[i] &&
         (rc = cuda_status(cudaMemcpyAsync(V1[i], h->V[i], bytes, cudaMemcpyDeviceToDevice, h->s),
                           "sns_ns_get_state")))
       return rc;
-    if (cross0 && cross0[i] &&
+    if (h->hist == HIST_FOURIER && cross0 && cross0[i] &&
         (rc = cuda_status(
              cudaMemcpyAsync(cross0[i], h->C0[i], bytes, cudaMemcpyDeviceToDevice, h->s),
              "sns_ns_get_state")))
       return rc;
+  }
+  if (h->hist != HIST_FOURIER && cross0) {
+    void *src[3], *dst[3];
+    int n = 0;
+    for (int i = 0; i < 3; i++)
+      if (cross0[i]) {
+        src[n] = h->hist == HIST_Z_U ? h->U[i] : h->C0[i];
+        dst[n++] = cross0[i];
+      }
+    if (n && (rc = ns_hist_fourier(h->pl, src, dst, n, h->s))) return rc;
   }
   if (omega1) {
     if (!vec_ok((const void* const*)omega1, "sns_ns_get_state")) return ERR_ARG;
@@ -1103,6 +1158,7 @@ int sns_ns_tune(sns_ns* h) {
   h->pl = q;
   drop_graph(h);
   h->carried = false;
+  h->hist = HIST_FOURIER;
   std::lock_guard<std::mutex> lock(g_tune_mu);
   g_tuned[key] = q;
   return OK;
@@ -1168,6 +1224,8 @@ int sns_ns_set_closure(sns_ns* h, int model, double cs_delta2, const void* mlp, 
       }
     }
   }
+  // the history with the cutoff it was made under
+  if (int rc = hist_to_fourier(h)) return rc;
   h->cl.model = model;
   h->cl.csd2 = cs_delta2;
   h->cl.mlp = mlp;

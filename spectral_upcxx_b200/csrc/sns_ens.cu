@@ -40,10 +40,11 @@ constexpr int kEnsMinLine = 16, kEnsMaxLine = 256;
 // Device-resident description of one box (the table is ordered by class).
 struct EnsBox {
   void* V[3];
-  void* C0[3];
+  void* C0[3];  // the history of the step (see UpdateArgs::C0)
   void* U[6];
   double* stats;  // per-tile diagnostics of the update stage
   double hK, nuhK;
+  const int* fourier;  // nonzero: the history is Fourier (its state was just set)
 };
 
 // Device-resident description of one box size within one stage.
@@ -56,7 +57,7 @@ struct EnsClass {
   int nf;         // fields of a line stage
   double scale2;  // 1/N^2 of the cross product
   const void* tw;
-  int pf_self;    // update stage: ask L2 for a tile's V and C0 once its cross
+  int pf_self;    // update stage: ask L2 for a tile's V once its cross
                   // product's loads are in flight
 };
 
@@ -118,6 +119,7 @@ __device__ __forceinline__ void ens_item(const EnsClass* __restrict__ k,
       a.hK = box->hK;
       a.nuhK = box->nuhK;
       a.stats = box->stats;
+      a.fourier = *box->fourier != 0;
       a.kc2 = 1e300;
       a.kx_half = 0;
       a.pf = 0;
@@ -261,7 +263,12 @@ struct sns_ens {
   std::vector<BoxHost> boxes;      // table order (grouped by class)
   std::vector<int> user_to_table;  // box index of the caller -> table index
   std::vector<ClassHost> classes;
+  // two box tables: the cross product is built in U[0..2] with the history in C0
+  // (turn 0) or the other way round (turn 1); steps take turns
   EnsBox* d_boxes = nullptr;
+  int turn = 0;
+  int* d_fourier = nullptr;   // per box (table order): its history is Fourier
+  std::vector<char> pending;  // the same on the host
   EnsClass* d_cls = nullptr;  // kEnsStages x nclass
   int64_t* d_parts_ens = nullptr;
   int64_t* d_parts_seq = nullptr;
@@ -270,8 +277,8 @@ struct sns_ens {
   EnsStage st[kEnsStages];
   int grid[kEnsStages];
   size_t smem[kEnsStages];
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  cudaGraph_t graph[2] = {};
+  cudaGraphExec_t exec[2] = {};
   int last_mode = -1;  // mode of the last step (selects the partial counts)
   bool stepped = false;
 };
@@ -413,7 +420,8 @@ int build_stage(sns_ens* e, int s, const StageCfg& cfg) {
 }
 
 int launch_stage(const sns_ens* e, int s, cudaStream_t stream) {
-  const EnsStage& st = e->st[s];
+  EnsStage st = e->st[s];
+  st.boxes += e->turn * e->boxes.size();
   const dim3 grid(e->grid[s]), block(e->cfg[s].threads);
   const size_t smem = e->smem[s];
   if (e->prec == PREC_C128) {
@@ -435,6 +443,32 @@ int launch_stage(const sns_ens* e, int s, cudaStream_t stream) {
   }
   SNS_CHECK_LAUNCH("k_ens_stage");
   return OK;
+}
+
+// After a step: the fields change places, and every history is this step's.
+int end_step(sns_ens* e) {
+  e->turn ^= 1;
+  bool any = false;
+  for (char& p : e->pending) {
+    any = any || p;
+    p = 0;
+  }
+  if (!any) return OK;
+  return cuda_status(cudaMemsetAsync(e->d_fourier, 0, sizeof(int) * e->boxes.size(), e->s),
+                     "sns_ens_step");
+}
+
+// The history fields of box i for the coming step, and the other three.
+void* const* history(const sns_ens* e, int i) {
+  return e->turn ? e->boxes[i].U : e->boxes[i].C0;
+}
+void* const* product(const sns_ens* e, int i) {
+  return e->turn ? e->boxes[i].C0 : e->boxes[i].U;
+}
+// The history of box i was set to Fourier fields.
+int mark_fourier(sns_ens* e, int i) {
+  e->pending[i] = 1;
+  return cuda_status(cudaMemsetAsync(e->d_fourier + i, 1, sizeof(int), e->s), "sns_ens_set_state");
 }
 
 int launch_step(const sns_ens* e, cudaStream_t stream) {
@@ -522,8 +556,10 @@ int configure(sns_ens* e, bool tune) {
 }
 
 void release(sns_ens* e) {
-  if (e->exec) cudaGraphExecDestroy(e->exec);
-  if (e->graph) cudaGraphDestroy(e->graph);
+  for (int i = 0; i < 2; i++) {
+    if (e->exec[i]) cudaGraphExecDestroy(e->exec[i]);
+    if (e->graph[i]) cudaGraphDestroy(e->graph[i]);
+  }
   for (BoxHost& b : e->boxes) {
     for (int d = 0; d < 3; d++) {
       pool_free(b.V[d]);
@@ -533,6 +569,7 @@ void release(sns_ens* e) {
     pool_free(b.stats);
   }
   pool_free(e->d_boxes);
+  pool_free(e->d_fourier);
   pool_free(e->d_cls);
   pool_free(e->d_parts_ens);
   pool_free(e->d_parts_seq);
@@ -647,12 +684,14 @@ int sns_ens_create(sns_ens** handle, int nboxes, const int64_t* dims, const doub
     if (!rc) rc = pool_malloc((void**)&b.stats, sizeof(double) * 4 * (size_t)b.nx * b.ny);
   }
   const int nb = (int)e->boxes.size(), nc = (int)e->classes.size();
-  if (!rc) rc = pool_malloc((void**)&e->d_boxes, sizeof(EnsBox) * nb);
+  if (!rc) rc = pool_malloc((void**)&e->d_boxes, sizeof(EnsBox) * 2 * nb);
+  if (!rc) rc = pool_malloc((void**)&e->d_fourier, sizeof(int) * nb);
+  e->pending.assign(nb, 0);
   if (!rc) rc = pool_malloc((void**)&e->d_cls, sizeof(EnsClass) * kEnsStages * nc);
   if (!rc) rc = pool_malloc((void**)&e->d_parts_ens, sizeof(int64_t) * nb);
   if (!rc) rc = pool_malloc((void**)&e->d_parts_seq, sizeof(int64_t) * nb);
   if (!rc) rc = pool_malloc((void**)&e->d_stats, sizeof(double) * 4 * nb);
-  std::vector<EnsBox> hb(nb);
+  std::vector<EnsBox> hb(2 * nb);
   std::vector<int64_t> seq_parts(nb);
   for (int i = 0; i < nb && !rc; i++) {
     const BoxHost& b = e->boxes[i];
@@ -664,16 +703,22 @@ int sns_ens_create(sns_ens** handle, int nboxes, const int64_t* dims, const doub
     hb[i].stats = b.stats;
     hb[i].hK = dt / 2;
     hb[i].nuhK = b.nu * dt / 2;
+    hb[i].fourier = e->d_fourier + i;
+    hb[nb + i] = hb[i];
+    for (int d = 0; d < 3; d++) std::swap(hb[nb + i].C0[d], hb[nb + i].U[d]);
     seq_parts[i] = e->classes[b.cls].seq.update_blocks;
   }
   if (!rc)
-    rc = cuda_status(cudaMemcpyAsync(e->d_boxes, hb.data(), sizeof(EnsBox) * nb,
+    rc = cuda_status(cudaMemcpyAsync(e->d_boxes, hb.data(), sizeof(EnsBox) * 2 * nb,
                                      cudaMemcpyHostToDevice, e->s),
                      "sns_ens_create");
   if (!rc)
     rc = cuda_status(cudaMemcpyAsync(e->d_parts_seq, seq_parts.data(), sizeof(int64_t) * nb,
                                      cudaMemcpyHostToDevice, e->s),
                      "sns_ens_create");
+  // the fields are zero: no history to transform, and what the tuner times
+  if (!rc)
+    rc = cuda_status(cudaMemsetAsync(e->d_fourier, 0, sizeof(int) * nb, e->s), "sns_ens_create");
   if (!rc) rc = cuda_status(cudaStreamSynchronize(e->s), "sns_ens_create");
   // kernels may use the device's full shared memory
   for (int s = 0; s < kEnsStages && !rc; s++) {
@@ -730,8 +775,12 @@ int sns_ens_bootstrap(sns_ens* e, int box, const void* const V0[3], const void* 
       !vec3(omega0, "sns_ens_bootstrap"))
     return ERR_ARG;
   BoxHost& b = e->boxes[e->user_to_table[box]];
+  const int i = e->user_to_table[box];
   const Dims d{(int)b.nx, (int)b.ny, (int)b.nz};
-  int rc = ns_bootstrap_fields(d, e->prec, b.nu, e->dt, V0, omega0, b.V, b.C0, b.U, e->s);
+  void* const* p = product(e, i);
+  void* const work[6] = {p[0], p[1], p[2], b.U[3], b.U[4], b.U[5]};
+  int rc = ns_bootstrap_fields(d, e->prec, b.nu, e->dt, V0, omega0, b.V, history(e, i), work, e->s);
+  if (!rc) rc = mark_fourier(e, i);
   if (rc) return rc;
   e->stepped = false;
   return OK;
@@ -747,10 +796,12 @@ int sns_ens_set_state(sns_ens* e, int box, const void* const V1[3], const void* 
     int rc = cuda_status(cudaMemcpyAsync(b.V[d], V1[d], bytes, cudaMemcpyDeviceToDevice, e->s),
                          "sns_ens_set_state");
     if (!rc)
-      rc = cuda_status(cudaMemcpyAsync(b.C0[d], cross0[d], bytes, cudaMemcpyDeviceToDevice, e->s),
+      rc = cuda_status(cudaMemcpyAsync(history(e, e->user_to_table[box])[d], cross0[d], bytes,
+                                       cudaMemcpyDeviceToDevice, e->s),
                        "sns_ens_set_state");
     if (rc) return rc;
   }
+  if (int rc = mark_fourier(e, e->user_to_table[box])) return rc;
   e->stepped = false;
   return OK;
 }
@@ -767,11 +818,34 @@ int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1
         (rc = cuda_status(cudaMemcpyAsync(V1[i], b.V[i], bytes, cudaMemcpyDeviceToDevice, e->s),
                           "sns_ens_get_state")))
       return rc;
-    if (cross0 && cross0[i] &&
-        (rc = cuda_status(cudaMemcpyAsync(cross0[i], b.C0[i], bytes, cudaMemcpyDeviceToDevice,
-                                          e->s),
-                          "sns_ens_get_state")))
+  }
+  if (cross0) {
+    const int t = e->user_to_table[box];
+    void *src[3], *dst[3];
+    int n = 0;
+    for (int i = 0; i < 3; i++)
+      if (cross0[i]) {
+        src[n] = history(e, t)[i];
+        dst[n++] = cross0[i];
+      }
+    // a history before its z-forward, or Fourier fields (or a destination that
+    // only a byte copy can write: through the product's fields, free here)
+    const bool fourier = e->pending[t] != 0;
+    for (int i = 0; i < n && !fourier; i++)
+      if (reinterpret_cast<uintptr_t>(dst[i]) % esize_of(e->prec)) dst[i] = product(e, t)[i];
+    if (n && !fourier &&
+        (rc = ns_hist_fourier(e->classes[b.cls].seq, src, dst, n, e->s)))
       return rc;
+    for (int i = 0, k = 0; i < 3; i++)
+      if (cross0[i]) {
+        const void* from = fourier ? src[k] : dst[k];
+        k++;
+        if (from != cross0[i] &&
+            (rc = cuda_status(cudaMemcpyAsync(cross0[i], from, bytes, cudaMemcpyDeviceToDevice,
+                                              e->s),
+                              "sns_ens_get_state")))
+          return rc;
+      }
   }
   if (omega1) {
     if (!vec3((const void* const*)omega1, "sns_ens_get_state")) return ERR_ARG;
@@ -791,8 +865,8 @@ int sns_ens_step(sns_ens* e, int nsteps, int mode) {
     return ERR_ARG;
   }
   int rc = OK;
-  if (mode == SNS_ENS_GRAPH && nsteps > 0 && !e->exec) {
-    // capture one ensemble step on the private stream, replayed on the caller's
+  // one ensemble step captured on the private stream, replayed on the caller's
+  auto capture = [&]() -> int {
     if ((rc = cuda_status(cudaStreamBeginCapture(e->cap, cudaStreamCaptureModeThreadLocal),
                           "sns_ens_step(capture)")))
       return rc;
@@ -803,27 +877,36 @@ int sns_ens_step(sns_ens* e, int nsteps, int mode) {
       if (g) cudaGraphDestroy(g);
       return lrc ? lrc : rc;
     }
-    if ((rc = cuda_status(cudaGraphInstantiate(&e->exec, g, 0), "sns_ens_step(instantiate)"))) {
+    if ((rc = cuda_status(cudaGraphInstantiate(&e->exec[e->turn], g, 0),
+                          "sns_ens_step(instantiate)"))) {
       cudaGraphDestroy(g);
-      e->exec = nullptr;
+      e->exec[e->turn] = nullptr;
       return rc;
     }
-    e->graph = g;
-  }
+    e->graph[e->turn] = g;
+    return OK;
+  };
   for (int t = 0; t < nsteps; t++) {
     if (mode == SNS_ENS_GRAPH) {
-      rc = cuda_status(cudaGraphLaunch(e->exec, e->s), "sns_ens_step(graph)");
+      if (!e->exec[e->turn] && (rc = capture())) return rc;
+      rc = cuda_status(cudaGraphLaunch(e->exec[e->turn], e->s), "sns_ens_step(graph)");
     } else if (mode == SNS_ENS_EAGER) {
       rc = launch_step(e, e->s);
     } else {
-      for (const BoxHost& b : e->boxes) {
+      for (int i = 0; i < (int)e->boxes.size(); i++) {
+        const BoxHost& b = e->boxes[i];
         void* V[3] = {b.V[0], b.V[1], b.V[2]};
-        void* C0[3] = {b.C0[0], b.C0[1], b.C0[2]};
-        void* U[6] = {b.U[0], b.U[1], b.U[2], b.U[3], b.U[4], b.U[5]};
-        rc = ns_step_once(e->classes[b.cls].seq, V, C0, U, b.stats, nullptr, b.nu, e->dt, e->s);
+        void* const* h = history(e, i);
+        void* const* p = product(e, i);
+        void* C0[3] = {h[0], h[1], h[2]};
+        void* U[6] = {p[0], p[1], p[2], b.U[3], b.U[4], b.U[5]};
+        int hist = e->pending[i] ? HIST_FOURIER : HIST_Z_C0;
+        rc = ns_step_once(e->classes[b.cls].seq, V, C0, U, b.stats, nullptr, b.nu, e->dt, e->s,
+                          nullptr, nullptr, nullptr, &hist);
         if (rc) break;
       }
     }
+    if (!rc) rc = end_step(e);
     if (rc) return rc;
     e->stepped = true;
     e->last_mode = mode;
@@ -891,6 +974,7 @@ int sns_ens_stage_times(sns_ens* e, int nsteps, double* ms) {
       rc = launch_stage(e, s, e->s);
       if (!rc) rc = cuda_status(cudaEventRecord(m[s + 1], e->s), "sns_ens_stage_times");
     }
+    if (!rc) rc = end_step(e);
     if (!rc) {
       e->stepped = true;
       e->last_mode = SNS_ENS_EAGER;

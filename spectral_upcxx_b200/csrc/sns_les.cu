@@ -431,6 +431,7 @@ int les_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* c
     a.C0[d] = C0[d];
   }
   for (int q = 0; q < 6; q++) a.tau[q] = U[3 + q];
+  a.fourier = 1;
   a.nx = nx;
   a.ny = ny;
   a.nz = nz;

@@ -1,7 +1,7 @@
 // Fused pseudo-spectral Navier-Stokes step (exec/ns.cpp:167-217).
 //
-// State: V (Fourier velocity, 3 fields) and C0 (Fourier V x omega of the
-// previous step, 3 fields); work: U (6 fields).  One step is five passes:
+// State: V (Fourier velocity, 3 fields) and C0 (V x omega of the previous step,
+// 3 fields); work: U (6 fields).  One step is five passes:
 //
 //   K1  z-inverse of (V, i k x V): the curl is formed while the tile loads
 //       (ns.cpp:206 + Vector::cross's inverse copies, src/Vector.cpp:74-77)
@@ -9,9 +9,15 @@
 //   K3  x-inverse, 1/N^2-scaled complex cross product u x omega, x-forward
 //       (src/Vector.cpp:79-89), 6 fields in, 3 out
 //   K4  y-forward of the 3 fields
-//   K5  z-forward + Nyquist zeroing (cross1 complete), then per mode the AB2 /
-//       projection / Crank-Nicolson update (ns.cpp:170-187) written over V,
-//       cross1 written over C0, FP64 diagnostics (ns.cpp:206-210)
+//   K5  z-forward of 3 cross1 - cross0 + Nyquist zeroing, then per mode the AB2 /
+//       projection / Crank-Nicolson update (ns.cpp:170-187) written over V, FP64
+//       diagnostics (ns.cpp:206-210)
+//
+// The history cross0 is kept as K4 left it, before its z-forward (the transform
+// is linear), so K5 reads nine fields and writes three: cross1 is neither
+// transformed on its own nor written.  U[0..2] and C0 take turns as the place
+// where a step builds its cross product and where its history is (HIST_Z_*);
+// a state that was just set has its Fourier history in C0.
 //
 // The reference runs 9 separate 3D FFTs plus ~25 eager field sweeps and 15
 // deep copies per step; here the history copies (ns.cpp:213-217) are
@@ -391,18 +397,57 @@ int run_k1(const NSPlan& pl, void* const V[3], void* const U[6], int* err_word, 
 
 }  // namespace
 
-int ns_k1_once(const NSPlan& pl, void* const V[3], void* const U[6], int* sync_words,
-               cudaStream_t s) {
+namespace {
+
+// The six fields a step works in: its cross product is built where its history
+// is not.
+struct StepFields {
+  void* U[6];
+  void* H[3];
+};
+StepFields step_fields(void* const C0[3], void* const U[6], int hist) {
+  StepFields f;
+  for (int i = 0; i < 3; i++) {
+    f.U[i] = hist == HIST_Z_U ? C0[i] : U[i];
+    f.H[i] = hist == HIST_Z_U ? U[i] : C0[i];
+    f.U[3 + i] = U[3 + i];
+  }
+  return f;
+}
+
+}  // namespace
+
+int ns_k1_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* const U[6], int hist,
+               int* sync_words, cudaStream_t s) {
   if (pl.k1_lines) {
     set_error("ns_k1_once: K1 as a line pass writes the work fields W, not U");
     return ERR_ARG;
   }
-  return run_k1(pl, V, U, sync_words ? sync_words + xy_sync_words(pl.nz) - 1 : nullptr, s);
+  return run_k1(pl, V, step_fields(C0, U, hist).U,
+                sync_words ? sync_words + xy_sync_words(pl.nz) - 1 : nullptr, s);
 }
 
-int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* const U[6],
+int ns_hist_fourier(const NSPlan& pl, void* const* src, void* const* dst, int n, cudaStream_t s) {
+  FieldPtrs f{};
+  f.n = n;
+  for (int i = 0; i < n; i++) {
+    f.in[i] = src[i];
+    f.out[i] = dst[i];
+  }
+  LineGeo g = axis_geo(2, pl.nx, pl.ny, pl.nz, pl.prec);
+  g.kx_half = pl.real;
+  int rc = run_line_pass(g, f, -1, PASS_ZERO_NYQUIST, 1.0, pl.prec, s);
+  for (int i = 0; i < n && !rc && pl.kc2 < 1e300; i++)
+    rc = op_cutoff(dst[i], pl.kc2, pl.real, Dims{pl.nx, pl.ny, pl.nz}, pl.prec, s);
+  return rc;
+}
+
+int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* const U_[6],
                  double* stats, int* sync_words, double nu, double dt, cudaStream_t s,
-                 cudaEvent_t* ev, void* const* W, bool* carried) {
+                 cudaEvent_t* ev, void* const* W, bool* carried, int* hist) {
+  const int h0 = hist ? *hist : HIST_FOURIER;
+  const StepFields sf = step_fields(C0, U_, h0);
+  void* const(&U)[6] = sf.U;
   const int nx = pl.nx, ny = pl.ny, nz = pl.nz, prec = pl.prec;
   // the error word of the step's bounded waits
   int* err_word = sync_words ? sync_words + xy_sync_words(nz) - 1 : nullptr;
@@ -523,8 +568,9 @@ int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* co
     for (int d = 0; d < 3; d++) {
       a.U[d] = U[d];
       a.V[d] = V[d];
-      a.C0[d] = C0[d];
+      a.C0[d] = sf.H[d];
     }
+    a.fourier = h0 == HIST_FOURIER;
     a.nx = nx;
     a.ny = ny;
     a.nz = nz;
@@ -537,15 +583,20 @@ int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* co
     a.kc2 = pl.kc2;
     a.kx_half = pl.real;
     if (carry) {
-      // K5 with the next step's K1 carried: U receives the z-inverse of the
-      // new V and of its curl
-      for (int i = 0; i < 6; i++) a.Uo[i] = U[i];
+      // K5 with the next step's K1 carried: the next step's fields receive the
+      // z-inverse of the new V and of its curl (over this step's history, which
+      // the tile has read)
+      for (int i = 0; i < 3; i++) {
+        a.Uo[i] = sf.H[i];
+        a.Uo[3 + i] = U[3 + i];
+      }
       rc = prec == PREC_C128 ? ns_update_carry<double>(pl, a, s) : ns_update_carry<float>(pl, a, s);
     } else {
       rc = ns_update(pl, a, false, s, err_word);
     }
     if (rc) return rc;
     if (carried) *carried = carry;
+    if (hist) *hist = h0 == HIST_Z_U ? HIST_Z_C0 : HIST_Z_U;
     mark();
   }
   return OK;
@@ -629,9 +680,10 @@ int ns_tune_plan(NSPlan& pl, void* const V[3], void* const C0[3], void* const U[
   auto measure = [&](const NSPlan& c, unsigned passes, float* out) -> int {
     float best = 3.4e38f;
     bool carried = false;
+    int hist = HIST_FOURIER;
     for (int r = 0; r < 6; r++) {
       int e = ns_step_once(c, V, C0, U, stats, sync_words, 0.0, 0.0, s, r ? ev : nullptr, W,
-                           &carried);
+                           &carried, &hist);
       if (e) return e;
       if (!r) continue;
       if ((e = cuda_status(cudaEventSynchronize(ev[kNSPasses]), "ns_tune_plan"))) return e;

@@ -77,15 +77,25 @@ bool ns_fits_l2(const NSPlan& pl);
 // true the step skips K1 (its pass time is then empty); on return it says
 // whether this step's K5 left the next step's K1 output in U.  Anything else
 // that writes V or U must clear it.
+// `hist` says where the history cross0 is and is updated: HIST_FOURIER, its
+// Fourier fields in C0 (a state just set); HIST_Z_C0 or HIST_Z_U, cross0 before
+// its z-forward in C0 or in U[0..2] (left there by the step before: a step
+// builds its cross product in the other three fields).  Null: HIST_FOURIER in
+// and nothing out.
+enum : int { HIST_FOURIER = 0, HIST_Z_C0 = 1, HIST_Z_U = 2 };
 constexpr int kNSPasses = 5;
 constexpr int kNSLineWork = 5;
 int ns_step_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* const U[6],
                  double* stats, int* sync_words, double nu, double dt, cudaStream_t s,
-                 cudaEvent_t* ev = nullptr, void* const* W = nullptr, bool* carried = nullptr);
+                 cudaEvent_t* ev = nullptr, void* const* W = nullptr, bool* carried = nullptr,
+                 int* hist = nullptr);
+// The Fourier history of a step state: dst = the z-forward of src (Nyquist planes
+// and modes beyond the cutoff zero) for the n fields given (dst may be src).
+int ns_hist_fourier(const NSPlan& pl, void* const* src, void* const* dst, int n, cudaStream_t s);
 // K1 alone (z-inverse of V and of i k x V into U[0..5]), for a carrying plan
 // whose U does not hold it yet (before a captured steady-state step).
-int ns_k1_once(const NSPlan& pl, void* const V[3], void* const U[6], int* sync_words,
-               cudaStream_t s);
+int ns_k1_once(const NSPlan& pl, void* const V[3], void* const C0[3], void* const U[6], int hist,
+               int* sync_words, cudaStream_t s);
 // The update pass (z-forward + AB2 / projection / CN update) on the fields of
 // `a`; sgs adds the divergence of the Fourier eddy stress a.tau.
 struct UpdateArgs;

@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 // product for a tile (W x L boxes) come into a shared-memory stage by TMA, and
 // the next tile's boxes are issued as soon as the current tile's threads have
 // read the stage into registers, so they load under the current tile's
-// transforms and update.  V and C0 are read in the update as before.  The
+// transforms and update.  V and the history are read as before.  The
 // diagnostics of each tile go to its own slot of a.stats, as in k_zfwd_update.
 // Bounded waits and the stall test as in k_zcurl_tma.
 template <typename T, int L>
@@ -437,6 +437,10 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
                                          const C* src = stage + fld * comp + j * W + w;
 #pragma unroll
                                          for (int e = 0; e < E; e++) v[e] = src[TPL * e * W];
+                                         if (!a.fourier) {
+                                           const int64_t nxy = (int64_t)a.nx * a.ny;
+                                           ab2_rows<E>(a, fld, blk * W + w + nxy * j, nxy * TPL, v);
+                                         }
                                          // every thread has read the stage: refill it
                                          __syncthreads();
                                          if (threadIdx.x == 0 && more) {

@@ -115,6 +115,17 @@ __global__ void k_vlaplacian(const cx_t<T>* __restrict__ v0, const cx_t<T>* __re
   }
 }
 
+template <typename T>
+__global__ void k_cutoff(cx_t<T>* f, double kc2, int kx_half, Dims d) {
+  const uint32_t n = (uint32_t)d.n();
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Idx p = decompose(i, d.nx, d.ny);
+    const double kx = kx_half ? p.x : freq_i(p.x, d.nx), ky = freq_i(p.y, d.ny),
+                 kz = freq_i(p.z, d.nz);
+    if (kx * kx + ky * ky + kz * kz > kc2) f[i] = mk((T)0, (T)0);
+  }
+}
+
 struct BootstrapArgs {
   const void* V0[3];
   const void* c0[3];
@@ -304,6 +315,16 @@ int op_laplacian_inverse(void* f, double a, double b, Dims d, int prec, cudaStre
   else
     k_laplacian_inverse<float><<<grid_for(d.n()), kThreads, 0, s>>>(mp<float>(f), a, b, d);
   SNS_CHECK_LAUNCH("k_laplacian_inverse");
+  return OK;
+}
+
+int op_cutoff(void* f, double kc2, bool kx_half, Dims d, int prec, cudaStream_t s) {
+  if (!dims_ok(d)) return ERR_ARG;
+  if (prec == PREC_C128)
+    k_cutoff<double><<<grid_for(d.n()), kThreads, 0, s>>>(mp<double>(f), kc2, kx_half, d);
+  else
+    k_cutoff<float><<<grid_for(d.n()), kThreads, 0, s>>>(mp<float>(f), kc2, kx_half, d);
+  SNS_CHECK_LAUNCH("k_cutoff");
   return OK;
 }
 

@@ -14,6 +14,8 @@ struct Dims {
 int op_gradient(const void* f, void* gx, void* gy, void* gz, Dims d, int prec, cudaStream_t s);
 int op_laplacian(const void* f, void* out, Dims d, int prec, cudaStream_t s);
 int op_laplacian_inverse(void* f, double a, double b, Dims d, int prec, cudaStream_t s);
+// zero the modes |k|^2 > kc2 (kx_half: stored x index = kx)
+int op_cutoff(void* f, double kc2, bool kx_half, Dims d, int prec, cudaStream_t s);
 int op_curl(const void* const in[3], void* const out[3], Dims d, int prec, cudaStream_t s);
 int op_divergence(const void* const in[3], void* out, Dims d, int prec, cudaStream_t s);
 int op_vlaplacian(const void* const in[3], void* const out[3], Dims d, int prec,

@@ -680,7 +680,13 @@ __device__ __forceinline__ void xcross_tile(const Fields& f, const cx_t<T>* __re
 struct UpdateArgs {
   const void* U[3];  // cross1 after x, y forward passes
   void* V[3];        // in: V1, out: V (new)
-  void* C0[3];       // in: cross0, out: cross1
+  // the history cross0, by `fourier`: 1 its Fourier fields; 0 cross0 as it came
+  // into its own step's update, after the x and y forward passes.  The
+  // z-forward is linear, so the tile then transforms 3 cross1 - cross0 at once
+  // and cross1 is not written: it stays in U as the next step's history.  With
+  // SGS: Fourier, in cross0, out cross1.
+  void* C0[3];
+  int fourier;
   int nx, ny, nz;
   int lx;         // log2(nx)
   int W;          // adjacent z lines per tile (may exceed nx: rows of the xy plane)
@@ -700,7 +706,7 @@ struct UpdateArgs {
   // the carried z-inverse pass (zfwd_update_curl_tile): out(0..2) = the new
   // V, out(3..5) = i k x V, both z-inverse-transformed
   void* Uo[6];
-  // ask L2 for this tile's V and C0 before its z-forward (0: no)
+  // ask L2 for this tile's V before its z-forward (0: no)
   int pf_self;
 };
 
@@ -748,6 +754,19 @@ __device__ __forceinline__ const void* update_field(const UpdateArgs& a, int f) 
   for (int q = 0; q < 6; q++)
     if (f == 3 + q) r = a.tau[q];
   return r;
+}
+
+// v = 3 v - history at the E elements of a z line of component d (step apart).
+template <int E, typename C>
+__device__ __forceinline__ void ab2_rows(const UpdateArgs& a, int d, int64_t i0, int64_t step,
+                                         C (&v)[E]) {
+  using T = decltype(v[0].x);
+  const C* __restrict__ h = reinterpret_cast<const C*>(d == 0 ? a.C0[0] : d == 1 ? a.C0[1] : a.C0[2]);
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const C c0 = h[i0 + e * step];
+    v[e] = mk(fma_rn((T)3, v[e].x, -c0.x), fma_rn((T)3, v[e].y, -c0.y));
+  }
 }
 
 // Tile `blk` holds the W z lines whose xy-plane offsets are blk*W .. blk*W+W-1.
@@ -823,12 +842,15 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
   int z = threadIdx.x >> wsh;
   int64_t idx = xy + nxy * z;
   const int64_t didx = nxy * dz;
+  const bool hist = SGS || a.fourier;  // cross0 joins here
   C V1n[3], c0n[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) c0n[d] = mk((T)0, (T)0);
   if (z < L) {
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       V1n[d] = Vp[d][idx];
-      c0n[d] = Cp[d][idx];
+      if (hist) c0n[d] = Cp[d][idx];
     }
   }
   __syncthreads();
@@ -844,7 +866,7 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         V1n[d] = Vp[d][idx + didx];
-        c0n[d] = Cp[d][idx + didx];
+        if (hist) c0n[d] = Cp[d][idx + didx];
       }
     }
     const T kz = (T)freq_i(z, a.nz);
@@ -873,6 +895,7 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
     }
     const T kk[3] = {kx, ky, kz};
     // F = K/2 (3 c1 - c0)                          (ns.cpp:171)
+    // (without `hist` the rows hold 3 c1 - c0 already)
     // lap1 = nu K/2 (-|k|^2 V1)                    (ns.cpp:174)
     // s = V1 + lap1 + F; G = div s / (-|k|^2)      (ns.cpp:177-178)
     // Vhalf = V1 + F - grad G; V = (Vhalf + lap1) / (1 + nu K/2 |k|^2)
@@ -881,8 +904,10 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
     C s[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      s[d].x = fma_rn(hK, fma_rn((T)3, c1[d].x, -c0[d].x), fma_rn(lc, V1[d].x, V1[d].x));
-      s[d].y = fma_rn(hK, fma_rn((T)3, c1[d].y, -c0[d].y), fma_rn(lc, V1[d].y, V1[d].y));
+      const C t = hist ? mk(fma_rn((T)3, c1[d].x, -c0[d].x), fma_rn((T)3, c1[d].y, -c0[d].y))
+                       : c1[d];
+      s[d].x = fma_rn(hK, t.x, fma_rn(lc, V1[d].x, V1[d].x));
+      s[d].y = fma_rn(hK, t.y, fma_rn(lc, V1[d].y, V1[d].y));
     }
     C g = mk(fma_rn(kz, s[2].x, fma_rn(ky, s[1].x, mul_rn(kx, s[0].x))),
              fma_rn(kz, s[2].y, fma_rn(ky, s[1].y, mul_rn(kx, s[0].y))));
@@ -898,7 +923,7 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
       if (cut) vv = mk((T)0, (T)0);
       Vn[d] = vv;
       Vp[d][idx] = vv;
-      Cp[d][idx] = c1[d];
+      if constexpr (SGS) Cp[d][idx] = c1[d];
       if constexpr (KEEP) sm[(d * W + w) * RS + pad_pos(z)] = vv;
     }
     // diagnostics of the new velocity: per-mode terms in T, sums in FP64;
@@ -964,16 +989,16 @@ __device__ __forceinline__ void zfwd_update_tile(const UpdateArgs& a,
     const int64_t i0 = base + w + nxy * j;
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = src[i0 + nxy * (TPL * e)];
+    if constexpr (!SGS) {
+      if (!a.fourier) ab2_rows<E>(a, fld, i0, nxy * TPL, v);
+    }
     if (!SGS && a.pf_self) {
-      // with the cross product's loads in flight, ask L2 for this tile's V
-      // and C0, so that the update's loads after the z-forward find them there
+      // with the cross product's loads in flight, ask L2 for this tile's V, so
+      // that the update's loads after the z-forward find it there
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
+      for (int d = 0; d < 3; d++)
         prefetch_lines<L>(reinterpret_cast<const char*>(a.V[d]), base, W, 1, 0, nxy,
                           (int)sizeof(C), nthr);
-        prefetch_lines<L>(reinterpret_cast<const char*>(a.C0[d]), base, W, 1, 0, nxy,
-                          (int)sizeof(C), nthr);
-      }
     }
     if (!SGS && a.pf > 0 && (blk + a.pf) * W < nxy) {
       // and tile blk + pf's cross product, V and C0
