@@ -726,20 +726,28 @@ struct Divisor {
     }
   }
 };
-// k2: a whole number below 2^24 (FP32).  The correctly rounded FP32 reciprocal
-// of an FP32 number is the FP64 one rounded once more (53 >= 2 x 24 + 2).
+// The hardware's FP32 reciprocal (1 ulp).
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// k2: a whole number below 2^24 (FP32).  The approximate reciprocal improved by
+// one Newton-Raphson step, r (2 - k2 r), whose remainder is exact in an FMA:
+// within 0.500001 ulp, as the FP64 reciprocal rounded to FP32 is.
 __device__ __forceinline__ Divisor<float> divisor_whole(float k2) {
-  return {k2, __frcp_rn(k2)};
+  const float r = rcp_approx(k2);
+  return {k2, fma_rn(fma_rn(-k2, r, 1.f), r, r)};
 }
 __device__ __forceinline__ Divisor<double> divisor_whole(double k2) { return {k2, 1.0 / k2}; }
-// den >= 1 in FP64.  FP32: one Newton step in FP64 from the FP32 reciprocal
-// (relative error about 2^-46 before the rounding to FP32).
+// den >= 1 in FP64.  FP32: one Newton-Raphson step in FP64 from the approximate
+// FP32 reciprocal (relative error about 2^-44 before the rounding to FP32).
 template <typename T>
 __device__ __forceinline__ Divisor<T> divisor_of(double den) {
   if constexpr (sizeof(T) == 8) {
     return {den, 1.0 / den};
   } else {
-    const double r0 = (double)__frcp_rn((float)den);
+    const double r0 = (double)rcp_approx((float)den);
     return {(T)den, (T)fma_rn(fma_rn(-den, r0, 1.0), r0, r0)};
   }
 }
@@ -839,7 +847,10 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
   const bool line_nyq = y == (a.ny >> 1) || (!a.kx_half && x == (a.nx >> 1));
   // half spectrum: each stored kx > 0 mode stands for itself and its conjugate
   const double wgt = (a.kx_half && x > 0) ? 2.0 : 1.0;
+  const bool cutoff = a.kc2 < 1e300;
   int z = threadIdx.x >> wsh;
+  const T len = (T)a.nz, step = (T)dz;
+  T kz = (T)freq_i(z, a.nz);
   int64_t idx = xy + nxy * z;
   const int64_t didx = nxy * dz;
   const bool hist = SGS || a.fourier;  // cross0 joins here
@@ -855,7 +866,7 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
   }
   __syncthreads();
 #pragma unroll 1
-  for (; z < L; z += dz, idx += didx) {
+  for (; z < L; z += dz, idx += didx, kz += step, kz -= kz > (T)(L >> 1) ? len : (T)0) {
     C V1[3], c0[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -869,15 +880,19 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
         if (hist) c0n[d] = Cp[d][idx + didx];
       }
     }
-    const T kz = (T)freq_i(z, a.nz);
     const T k2 = fma_rn(kz, kz, kxy2);
     const double k2d = (double)k2;
     // modes beyond the cutoff are not evolved (zero velocity and history)
-    const bool cut = k2d > a.kc2;
+    const bool cut = cutoff && k2d > a.kc2;
     const bool nyq = cut || line_nyq || z == (a.nz >> 1);
     C c1[3];
+    const C* row0 = sm + w * RS + pad_pos(z);
 #pragma unroll
-    for (int d = 0; d < 3; d++) c1[d] = nyq ? mk((T)0, (T)0) : sm[(d * W + w) * RS + pad_pos(z)];
+    for (int d = 0; d < 3; d++) c1[d] = row0[d * W * RS];
+    if (nyq) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) c1[d] = mk((T)0, (T)0);
+    }
     if constexpr (SGS) {
       const T ws = (T)fmin(1.0, fmax(0.0, (sqrt(k2d) - a.sgs_klo) * a.sgs_kinv));
       if (!nyq && ws > (T)0) {
@@ -920,7 +935,7 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       C vv = mk(by_cn.under(fma_rn(-kk[d], g.x, s[d].x)), by_cn.under(fma_rn(-kk[d], g.y, s[d].y)));
-      if (cut) vv = mk((T)0, (T)0);
+      if (cutoff && cut) vv = mk((T)0, (T)0);
       Vn[d] = vv;
       Vp[d][idx] = vv;
       if constexpr (SGS) Cp[d][idx] = c1[d];
