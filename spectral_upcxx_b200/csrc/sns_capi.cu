@@ -805,16 +805,10 @@ int sns_ns_set_state(sns_ns* h, const void* const V1[3], const void* const cross
     return OK;
   }
   const size_t bytes = esize(h->pl.prec) * (size_t)h->pl.nx * h->pl.ny * h->pl.nz;
-  int rc;
-  for (int d = 0; d < 3; d++) {
-    if ((rc = cuda_status(cudaMemcpyAsync(h->V[d], V1[d], bytes, cudaMemcpyDeviceToDevice, h->s),
-                          "sns_ns_set_state")))
-      return rc;
-    if ((rc = cuda_status(
-             cudaMemcpyAsync(h->C0[d], cross0[d], bytes, cudaMemcpyDeviceToDevice, h->s),
-             "sns_ns_set_state")))
-      return rc;
-  }
+  const void* src[6] = {V1[0], V1[1], V1[2], cross0[0], cross0[1], cross0[2]};
+  void* dst[6] = {h->V[0], h->V[1], h->V[2], h->C0[0], h->C0[1], h->C0[2]};
+  int rc = op_copy_fields(src, dst, 6, bytes, h->s);
+  if (rc) return rc;
   h->stepped = false;
   h->carried = false;
   h->hist = HIST_FOURIER;
@@ -1003,16 +997,29 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
   for (int i = 0; i < 3 && cross0; i++)
     if (reinterpret_cast<uintptr_t>(cross0[i]) % esize(h->pl.prec))
       if ((rc = hist_to_fourier(h))) return rc;
-  for (int i = 0; i < 3; i++) {
-    if (V1 && V1[i] &&
-        (rc = cuda_status(cudaMemcpyAsync(V1[i], h->V[i], bytes, cudaMemcpyDeviceToDevice, h->s),
-                          "sns_ns_get_state")))
-      return rc;
-    if (h->hist == HIST_FOURIER && cross0 && cross0[i] &&
-        (rc = cuda_status(
-             cudaMemcpyAsync(cross0[i], h->C0[i], bytes, cudaMemcpyDeviceToDevice, h->s),
-             "sns_ns_get_state")))
-      return rc;
+  // V1 and its curl from one read of V where both are wanted
+  bool both = omega1 && V1 && V1[0] && V1[1] && V1[2];
+  for (int i = 0; i < 3 && both; i++)
+    both = omega1[i] && reinterpret_cast<uintptr_t>(V1[i]) % esize(h->pl.prec) == 0;
+  if (both) {
+    const void* v[3] = {h->V[0], h->V[1], h->V[2]};
+    if ((rc = op_curl_copy(v, V1, omega1, d, h->pl.prec, h->s))) return rc;
+  }
+  {
+    const void* src[6];
+    void* dst[6];
+    int n = 0;
+    for (int i = 0; i < 3; i++) {
+      if (!both && V1 && V1[i]) {
+        src[n] = h->V[i];
+        dst[n++] = V1[i];
+      }
+      if (h->hist == HIST_FOURIER && cross0 && cross0[i]) {
+        src[n] = h->C0[i];
+        dst[n++] = cross0[i];
+      }
+    }
+    if (n && (rc = op_copy_fields(src, dst, n, bytes, h->s))) return rc;
   }
   if (h->hist != HIST_FOURIER && cross0) {
     void *src[3], *dst[3];
@@ -1024,7 +1031,7 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
       }
     if (n && (rc = ns_hist_fourier(h->pl, src, dst, n, h->s))) return rc;
   }
-  if (omega1) {
+  if (omega1 && !both) {
     if (!vec_ok((const void* const*)omega1, "sns_ns_get_state")) return ERR_ARG;
     const void* v[3] = {h->V[0], h->V[1], h->V[2]};
     if ((rc = op_curl(v, omega1, d, h->pl.prec, h->s))) return rc;

@@ -803,15 +803,10 @@ int sns_ens_set_state(sns_ens* e, int box, const void* const V1[3], const void* 
     return ERR_ARG;
   BoxHost& b = e->boxes[e->user_to_table[box]];
   const size_t bytes = esize_of(e->prec) * (size_t)b.nx * b.ny * b.nz;
-  for (int d = 0; d < 3; d++) {
-    int rc = cuda_status(cudaMemcpyAsync(b.V[d], V1[d], bytes, cudaMemcpyDeviceToDevice, e->s),
-                         "sns_ens_set_state");
-    if (!rc)
-      rc = cuda_status(cudaMemcpyAsync(history(e, e->user_to_table[box])[d], cross0[d], bytes,
-                                       cudaMemcpyDeviceToDevice, e->s),
-                       "sns_ens_set_state");
-    if (rc) return rc;
-  }
+  void* const* h = history(e, e->user_to_table[box]);
+  const void* src[6] = {V1[0], V1[1], V1[2], cross0[0], cross0[1], cross0[2]};
+  void* dst[6] = {b.V[0], b.V[1], b.V[2], h[0], h[1], h[2]};
+  if (int rc = op_copy_fields(src, dst, 6, bytes, e->s)) return rc;
   if (int rc = mark_fourier(e, e->user_to_table[box])) return rc;
   e->stepped = false;
   return OK;
@@ -824,11 +819,19 @@ int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1
   const Dims d{(int)b.nx, (int)b.ny, (int)b.nz};
   const size_t bytes = esize_of(e->prec) * (size_t)d.n();
   int rc;
-  for (int i = 0; i < 3; i++) {
-    if (V1 && V1[i] &&
-        (rc = cuda_status(cudaMemcpyAsync(V1[i], b.V[i], bytes, cudaMemcpyDeviceToDevice, e->s),
-                          "sns_ens_get_state")))
-      return rc;
+  // V1 and its curl from one read of V where both are wanted
+  bool both = omega1 && V1 && V1[0] && V1[1] && V1[2];
+  for (int i = 0; i < 3 && both; i++)
+    both = omega1[i] && reinterpret_cast<uintptr_t>(V1[i]) % esize_of(e->prec) == 0;
+  if (both) {
+    const void* v[3] = {b.V[0], b.V[1], b.V[2]};
+    if ((rc = op_curl_copy(v, V1, omega1, d, e->prec, e->s))) return rc;
+  } else {
+    for (int i = 0; i < 3; i++)
+      if (V1 && V1[i] &&
+          (rc = cuda_status(cudaMemcpyAsync(V1[i], b.V[i], bytes, cudaMemcpyDeviceToDevice, e->s),
+                            "sns_ens_get_state")))
+        return rc;
   }
   if (cross0) {
     const int t = e->user_to_table[box];
@@ -858,7 +861,7 @@ int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1
           return rc;
       }
   }
-  if (omega1) {
+  if (omega1 && !both) {
     if (!vec3((const void* const*)omega1, "sns_ens_get_state")) return ERR_ARG;
     const void* v[3] = {b.V[0], b.V[1], b.V[2]};
     if ((rc = op_curl(v, omega1, d, e->prec, e->s))) return rc;

@@ -91,6 +91,35 @@ __global__ void k_curl(const cx_t<T>* __restrict__ v0, const cx_t<T>* __restrict
 }
 
 template <typename T>
+__global__ void k_curl_copy(const cx_t<T>* __restrict__ v0, const cx_t<T>* __restrict__ v1,
+                            const cx_t<T>* __restrict__ v2, cx_t<T>* p0, cx_t<T>* p1, cx_t<T>* p2,
+                            cx_t<T>* o0, cx_t<T>* o1, cx_t<T>* o2, Dims d) {
+  const uint32_t n = (uint32_t)d.n();
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Idx p = decompose(i, d.nx, d.ny);
+    const T kx = (T)freq_i(p.x, d.nx), ky = (T)freq_i(p.y, d.ny), kz = (T)freq_i(p.z, d.nz);
+    const cx_t<T> a = v0[i], b = v1[i], c = v2[i];
+    p0[i] = a;
+    p1[i] = b;
+    p2[i] = c;
+    o0[i] = csub(ikmul(ky, c), ikmul(kz, b));
+    o1[i] = csub(ikmul(kz, a), ikmul(kx, c));
+    o2[i] = csub(ikmul(kx, b), ikmul(ky, a));
+  }
+}
+
+struct CopyArgs {
+  const uint4* src[6];
+  uint4* dst[6];
+};
+__global__ void k_copy_fields(const CopyArgs a, uint32_t n16) {
+  const uint4* __restrict__ s = a.src[blockIdx.y];
+  uint4* __restrict__ d = a.dst[blockIdx.y];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += gridDim.x * blockDim.x)
+    d[i] = s[i];
+}
+
+template <typename T>
 __global__ void k_divergence(const cx_t<T>* __restrict__ v0, const cx_t<T>* __restrict__ v1,
                              const cx_t<T>* __restrict__ v2, cx_t<T>* out, Dims d) {
   const uint32_t n = (uint32_t)d.n();
@@ -315,6 +344,49 @@ int op_laplacian_inverse(void* f, double a, double b, Dims d, int prec, cudaStre
   else
     k_laplacian_inverse<float><<<grid_for(d.n()), kThreads, 0, s>>>(mp<float>(f), a, b, d);
   SNS_CHECK_LAUNCH("k_laplacian_inverse");
+  return OK;
+}
+
+int op_copy_fields(const void* const* src, void* const* dst, int n, size_t bytes, cudaStream_t s) {
+  // up to 32 MB a field one launch for all (a small copy takes the GPU about as
+  // long as a launch: set and read-back of a 32^3 state 19 us of twelve copies);
+  // larger ones, and unaligned ones, a copy each
+  bool one = n > 1 && n <= 6 && bytes % 16 == 0 && bytes <= (32u << 20);
+  for (int i = 0; i < n && one; i++)
+    one = reinterpret_cast<uintptr_t>(src[i]) % 16 == 0 &&
+          reinterpret_cast<uintptr_t>(dst[i]) % 16 == 0;
+  if (!one) {
+    for (int i = 0; i < n; i++) {
+      const int rc = cuda_status(cudaMemcpyAsync(dst[i], src[i], bytes, cudaMemcpyDeviceToDevice, s),
+                                 "field copy");
+      if (rc) return rc;
+    }
+    return OK;
+  }
+  CopyArgs a{};
+  for (int i = 0; i < n; i++) {
+    a.src[i] = static_cast<const uint4*>(src[i]);
+    a.dst[i] = static_cast<uint4*>(dst[i]);
+  }
+  const uint32_t n16 = (uint32_t)(bytes / 16);
+  k_copy_fields<<<dim3(grid_for(n16), n), kThreads, 0, s>>>(a, n16);
+  SNS_CHECK_LAUNCH("k_copy_fields");
+  return OK;
+}
+
+int op_curl_copy(const void* const v[3], void* const copy[3], void* const out[3], Dims d, int prec,
+                 cudaStream_t s) {
+  if (!dims_ok(d)) return ERR_ARG;
+  if (prec == PREC_C128)
+    k_curl_copy<double><<<grid_for(d.n()), kThreads, 0, s>>>(
+        cp<double>(v[0]), cp<double>(v[1]), cp<double>(v[2]), mp<double>(copy[0]),
+        mp<double>(copy[1]), mp<double>(copy[2]), mp<double>(out[0]), mp<double>(out[1]),
+        mp<double>(out[2]), d);
+  else
+    k_curl_copy<float><<<grid_for(d.n()), kThreads, 0, s>>>(
+        cp<float>(v[0]), cp<float>(v[1]), cp<float>(v[2]), mp<float>(copy[0]), mp<float>(copy[1]),
+        mp<float>(copy[2]), mp<float>(out[0]), mp<float>(out[1]), mp<float>(out[2]), d);
+  SNS_CHECK_LAUNCH("k_curl_copy");
   return OK;
 }
 

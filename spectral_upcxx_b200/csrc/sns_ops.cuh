@@ -14,6 +14,12 @@ struct Dims {
 int op_gradient(const void* f, void* gx, void* gy, void* gz, Dims d, int prec, cudaStream_t s);
 int op_laplacian(const void* f, void* out, Dims d, int prec, cudaStream_t s);
 int op_laplacian_inverse(void* f, double a, double b, Dims d, int prec, cudaStream_t s);
+// dst[i] = src[i] for n <= 6 fields of `bytes` bytes each, in one launch where the
+// fields are small (any alignment is taken)
+int op_copy_fields(const void* const* src, void* const* dst, int n, size_t bytes, cudaStream_t s);
+// copy = v and out = i k x v from one read of v
+int op_curl_copy(const void* const v[3], void* const copy[3], void* const out[3], Dims d, int prec,
+                 cudaStream_t s);
 // zero the modes |k|^2 > kc2 (kx_half: stored x index = kx)
 int op_cutoff(void* f, double kc2, bool kx_half, Dims d, int prec, cudaStream_t s);
 int op_curl(const void* const in[3], void* const out[3], Dims d, int prec, cudaStream_t s);
