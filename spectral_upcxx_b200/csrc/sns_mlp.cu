@@ -29,14 +29,28 @@ namespace sns {
 constexpr int kPart = kMlpParams + 1;  // gradients + loss sum
 
 // grad[p] = sum over CTAs of part[cta][p] (fixed order); the loss entry is
-// turned into the batch mean.
-__global__ void k_mlp_reduce(const float* __restrict__ part, int nblocks, float inv_batch,
-                             float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kPart) return;
+// turned into the batch mean.  A block takes 32 parameters, 16 slices of
+// the CTAs each, so that the 6.3 MB of partials are read by 166 blocks with many
+// loads in flight (one thread per parameter walked 296 partials one after the
+// other: 9.4 us on B200, now 4 us).
+constexpr int kReduceSlices = 16;
+__global__ void __launch_bounds__(32 * kReduceSlices)
+    k_mlp_reduce(const float* __restrict__ part, int nblocks, float inv_batch,
+                 float* __restrict__ grad) {
+  __shared__ float sm[kReduceSlices][33];
+  const int p = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
-  for (int b = 0; b < nblocks; b++) s += part[(int64_t)b * kPart + p];
-  grad[p] = p == kMlpParams ? s * inv_batch : s;
+  if (p < kPart) {
+#pragma unroll 8
+    for (int b = threadIdx.y; b < nblocks; b += kReduceSlices) s += part[(int64_t)b * kPart + p];
+  }
+  sm[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && p < kPart) {
+#pragma unroll
+    for (int y = 1; y < kReduceSlices; y++) s += sm[y][threadIdx.x];
+    grad[p] = p == kMlpParams ? s * inv_batch : s;
+  }
 }
 
 // Adam (bias-corrected) on the FP32 masters; writes the bf16 inference copy.
@@ -270,9 +284,11 @@ __global__ void __launch_bounds__(kTcRows)
 //   M5  dW1 += dPre1^T X (M 64, N 16)                   D cols 192..207
 // dW1 and dW2 accumulate in tensor memory over all the CTA's tiles (M = 64
 // accumulators: row r in lane 32 (r / 16) + r % 16).  The vector gradients
-// (db1, db2, dw3) are FP32 sums over samples, reduced across each warp by a
-// shuffle reduce-scatter (lane l keeps columns 2l, 2l + 1) and across warps
-// in a fixed order at the end; the scalars (db3, loss) likewise.  Rounding
+// (db1, db2, dw3) are FP32 sums over samples: per tile lanes l and l + 16
+// exchange halves of the columns and add to 32 running sums a vector, which
+// are reduced across the lanes and warps in a fixed order at the end (a full
+// reduce-scatter of every tile took 62 shuffles a vector instead of 32; 2^18
+// samples on B200: 49 us, now 46 us); the scalars (db3, loss) likewise.  Rounding
 // points as in the oracle: dPre2 and dPre1 enter the MMAs in BF16, the
 // vector sums use their FP32 values.  The CTA writes one partial (kPart
 // floats) for the deterministic reduce.
@@ -297,28 +313,44 @@ struct __align__(128) GradTcSmem {
   int abort;
 };
 // at most two CTAs per SM (2 x 256 tensor-memory columns): reserve enough
-// shared memory that a third never shares the SM
+// shared memory that a third never shares the SM.  (Three CTAs of 128 + 32
+// columns, M1 to M3 in the same ones, measured 50.7 us against 46.0: 168
+// registers spill and 2048 tiles make 4.6 rounds of 444 CTAs.)
 constexpr int kGtSmemBytes = 80 * 1024;
 static_assert(sizeof(GradTcSmem) <= kGtSmemBytes, "training tile fits the reservation");
 
-// Sum of v[c] over the 32 lanes of the warp for c = 0..63; lane l returns the
-// sums of columns 2l and 2l + 1.
-__device__ __forceinline__ void warp_colsum64(float (&v)[64], float& c0, float& c1) {
+// Running column sums of the warp's samples: v holds columns c0 .. c0 + 15 of
+// this lane's sample; lanes below 16 keep columns c0 .. c0 + 7, the others
+// c0 + 8 .. c0 + 15, in acc[c0 / 2 ..].
+__device__ __forceinline__ void colsum_add(const float (&v)[16], float (&acc)[32], int c0) {
+  const bool up = threadIdx.x & 16;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const float send = up ? v[i] : v[8 + i];
+    const float keep = up ? v[8 + i] : v[i];
+    acc[c0 / 2 + i] += keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+}
+// The sums over the half-warps' lanes into out[64]: lane l holds entries
+// 2 (l % 16) and the next of its half's 32.
+__device__ __forceinline__ void colsum_store(float (&acc)[32], float* out) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int o = 16, n = 32; o >= 1; o >>= 1, n >>= 1) {
+  for (int o = 8, n = 16; o >= 1; o >>= 1, n >>= 1) {
     const bool up = lane & o;
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
+    for (int i = 0; i < 16; i++) {
       if (i < n) {
-        const float send = up ? v[i] : v[n + i];
-        const float keep = up ? v[n + i] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        const float send = up ? acc[i] : acc[n + i];
+        const float keep = up ? acc[n + i] : acc[i];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
     }
   }
-  c0 = v[0];
-  c1 = v[1];
+  const int q = 2 * (lane & 15);
+  const int c = 16 * (q / 8) + 8 * (lane >> 4) + q % 8;
+  out[c] = acc[0];
+  out[c + 1] = acc[1];
 }
 
 __device__ __forceinline__ bool tc_step(uint64_t* mbar, uint32_t& phase, int& abort_flag) {
@@ -330,7 +362,7 @@ __device__ __forceinline__ bool tc_step(uint64_t* mbar, uint32_t& phase, int& ab
   return !abort_flag;
 }
 
-__global__ void __launch_bounds__(kGtRows)
+__global__ void __launch_bounds__(kGtRows, 2)
     k_mlp_grad_tc(const MlpPacked* __restrict__ P, const __nv_bfloat16* __restrict__ X,
                   const float* __restrict__ target, const float* __restrict__ weight,
                   const int* __restrict__ idx, int64_t B, float inv_batch,
@@ -387,7 +419,9 @@ __global__ void __launch_bounds__(kGtRows)
   constexpr uint32_t id_dw2 = tc::idesc_bf16(64, kMlpHidden, true, true);   // M4
   constexpr uint32_t id_dw1 = tc::idesc_bf16(64, kMlpK1, true, true);       // M5
   uint32_t phase = 0;
-  float acc_db1[2] = {0.f, 0.f}, acc_db2[2] = {0.f, 0.f}, acc_dw3[2] = {0.f, 0.f};
+  float acc_db1[32], acc_db2[32], acc_dw3[32];
+#pragma unroll
+  for (int i = 0; i < 32; i++) acc_db1[i] = acc_db2[i] = acc_dw3[i] = 0.f;
   float acc_db3 = 0.f, acc_loss = 0.f;
   bool first = true;
   const int64_t tiles = (B + kGtRows - 1) / kGtRows;
@@ -482,33 +516,26 @@ __global__ void __launch_bounds__(kGtRows)
       acc_loss += wt * d * d;
       dz = 2.f * inv_batch * wt * d / (1.f + expf(-z));
     }
-    float vw3[64], vb2[64];
 #pragma unroll
     for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
       uint32_t r[16];
       tc::tmem_ld16(tmem + lane_base + 64 + c0, r);
       uint32_t h[8];
+      float vw3[16], vb2[16];
 #pragma unroll
       for (int j = 0; j < 16; j++) {
         const float p2 = __uint_as_float(r[j]);
-        vw3[c0 + j] = dz * fmaxf(p2, 0.f);
-        vb2[c0 + j] = p2 > 0.f ? dz * S.w3[c0 + j] : 0.f;
+        vw3[j] = dz * fmaxf(p2, 0.f);
+        vb2[j] = p2 > 0.f ? dz * S.w3[c0 + j] : 0.f;
       }
 #pragma unroll
-      for (int j = 0; j < 8; j++) h[j] = pack_bf16(vb2[c0 + 2 * j], vb2[c0 + 2 * j + 1]);
+      for (int j = 0; j < 8; j++) h[j] = pack_bf16(vb2[2 * j], vb2[2 * j + 1]);
       *reinterpret_cast<uint4*>(S.P2 + tc::kmajor_off(tid, c0, kMlpHidden)) =
           make_uint4(h[0], h[1], h[2], h[3]);
       *reinterpret_cast<uint4*>(S.P2 + tc::kmajor_off(tid, c0 + 8, kMlpHidden)) =
           make_uint4(h[4], h[5], h[6], h[7]);
-    }
-    {
-      float a0, a1;
-      warp_colsum64(vw3, a0, a1);
-      acc_dw3[0] += a0;
-      acc_dw3[1] += a1;
-      warp_colsum64(vb2, a0, a1);
-      acc_db2[0] += a0;
-      acc_db2[1] += a1;
+      colsum_add(vw3, acc_dw3, c0);
+      colsum_add(vb2, acc_db2, c0);
     }
     {
       float d3 = dz;
@@ -535,27 +562,23 @@ __global__ void __launch_bounds__(kGtRows)
     if (!tc_step(&S.mbar, phase, S.abort)) break;
     // dPre1 = dH1 * (pre1 > 0) -> P1, db1
     {
-      float vb1[64];
 #pragma unroll
       for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
         uint32_t r[16];
         tc::tmem_ld16(tmem + lane_base + c0, r);
         uint32_t h[8];
+        float vb1[16];
 #pragma unroll
         for (int j = 0; j < 16; j++)
-          vb1[c0 + j] = ((mask1[(c0 + j) >> 5] >> ((c0 + j) & 31)) & 1u) ? __uint_as_float(r[j])
-                                                                          : 0.f;
+          vb1[j] = ((mask1[(c0 + j) >> 5] >> ((c0 + j) & 31)) & 1u) ? __uint_as_float(r[j]) : 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; j++) h[j] = pack_bf16(vb1[c0 + 2 * j], vb1[c0 + 2 * j + 1]);
+        for (int j = 0; j < 8; j++) h[j] = pack_bf16(vb1[2 * j], vb1[2 * j + 1]);
         *reinterpret_cast<uint4*>(S.P1 + tc::kmajor_off(tid, c0, kMlpHidden)) =
             make_uint4(h[0], h[1], h[2], h[3]);
         *reinterpret_cast<uint4*>(S.P1 + tc::kmajor_off(tid, c0 + 8, kMlpHidden)) =
             make_uint4(h[4], h[5], h[6], h[7]);
+        colsum_add(vb1, acc_db1, c0);
       }
-      float a0, a1;
-      warp_colsum64(vb1, a0, a1);
-      acc_db1[0] += a0;
-      acc_db1[1] += a1;
     }
     // M5 (dW1 += dPre1^T X)
     tc::fence_async_smem();
@@ -599,12 +622,9 @@ __global__ void __launch_bounds__(kGtRows)
         for (int j = 0; j < 16; j++)
           out[kMlpOffW1 + n * kMlpK1 + j] = (first || j >= kMlpIn) ? 0.f : __uint_as_float(r[j]);
     }
-    S.vec[warp][0][2 * lane] = acc_db1[0];
-    S.vec[warp][0][2 * lane + 1] = acc_db1[1];
-    S.vec[warp][1][2 * lane] = acc_db2[0];
-    S.vec[warp][1][2 * lane + 1] = acc_db2[1];
-    S.vec[warp][2][2 * lane] = acc_dw3[0];
-    S.vec[warp][2][2 * lane + 1] = acc_dw3[1];
+    colsum_store(acc_db1, S.vec[warp][0]);
+    colsum_store(acc_db2, S.vec[warp][1]);
+    colsum_store(acc_dw3, S.vec[warp][2]);
     float l = acc_loss;
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
@@ -676,8 +696,8 @@ int grad_launch(const void* packed, const void* X, const float* t, const float* 
       idx, B, inv, reinterpret_cast<float*>(part));
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
-    k_mlp_reduce<<<(kPart + 255) / 256, 256, 0, s>>>(reinterpret_cast<float*>(part), nb, inv,
-                                                    grad);
+    k_mlp_reduce<<<(kPart + 31) / 32, dim3(32, kReduceSlices), 0, s>>>(
+        reinterpret_cast<float*>(part), nb, inv, grad);
     e = cudaGetLastError();
   }
   // the pool may hand the block to any later caller: wait for the kernels
