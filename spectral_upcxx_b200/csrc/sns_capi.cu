@@ -405,6 +405,7 @@ int sns_version(void) { return 1; }
 int sns_malloc(void** ptr, size_t bytes) { return pool_malloc(ptr, bytes); }
 int sns_free(void* ptr) { return pool_free(ptr); }
 int sns_pool_trim(void) {
+  particles_trim();
   Pool& p = pool();
   std::lock_guard<std::mutex> lock(p.mu);
   return trim_locked(p);

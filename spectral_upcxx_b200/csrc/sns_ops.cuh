@@ -48,6 +48,9 @@ int op_average_abs(const void* f, int64_t n, int prec, double* partials, double*
                    cudaStream_t s);
 int reduce_partials_count();
 
+// Give back the workspace that ordered particle moves keep.
+void particles_trim();
+
 // Vector::cross on device fields (src/Vector.cpp:66-90) with six caller-given
 // work fields; tw_axes optionally supplies the twiddle table of each axis.
 int vector_cross(const void* const a[3], const void* const b[3], void* const out[3], Dims d,
