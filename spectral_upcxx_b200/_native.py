@@ -157,13 +157,23 @@ def check(fn: str, rc: int) -> int:
     return rc
 
 
+_FNS = {}
+
+
 def call(fn: str, *args) -> int:
-    return check(fn, getattr(lib(), fn)(*args))
+    f = _FNS.get(fn)
+    if f is None:
+        f = _FNS[fn] = getattr(lib(), fn)
+    rc = f(*args)
+    return rc if rc == SNS_OK else check(fn, rc)
+
+
+_VP3 = C.c_void_p * 3
 
 
 def ptr3(ptrs):
-    return (C.c_void_p * 3)(*[C.c_void_p(int(p)) for p in ptrs])
+    return _VP3(*ptrs)
 
 
 def ptrs(ps):
-    return (C.c_void_p * len(ps))(*[C.c_void_p(int(p)) for p in ps])
+    return (C.c_void_p * len(ps))(*ps)
