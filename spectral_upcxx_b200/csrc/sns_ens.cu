@@ -343,6 +343,7 @@ bool make_class(const sns_ens* e, int s, int c, const StageCfg& cfg, EnsClass& k
       g.sa = W;
       g.sb = (int64_t)G * nxy;
     }
+    g.run = field_run(g.TA * g.TB);
     k.L = L;
     k.W = W;
     k.G = G;

@@ -295,6 +295,7 @@ LineGeo axis_geo(int axis, int nx, int ny, int nz, int prec, int wmax, int tmax,
     g.sa = g.W;
     g.sb = (int64_t)g.G * nx;
   }
+  g.run = field_run(g.TA * g.TB);
   return g;
 }
 

@@ -74,9 +74,7 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
   // the fields are written by the pass before
   pdl_wait();
   auto issue = [&](int64_t b, int k) {  // thread 0
-    const int64_t blk = tile_order(b, ntiles, geo.rev);
-    const int fld = (int)(blk % nf);
-    const int64_t t = blk / nf;
+    const auto [fld, t] = line_slot(geo.run, tile_order(b, ntiles, geo.rev), nf);
     const CUtensorMap* m = pick_map(fld, m0, m1, m2, m3, m4, m5);
     const int u = (int)(sizeof(C) / 8);
     C* st = stage0 + k * per;

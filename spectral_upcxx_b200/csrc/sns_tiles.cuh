@@ -27,25 +27,29 @@ namespace sns {
 // between radix stages.
 struct LineCoord {
   int64_t idx0, step;  // global index of position j, stride between e
-  int x, y, z;         // coordinates of position j (3D fields)
+  int x, y, z;         // coordinates of position j (y and z lines of 3D fields)
 };
 
-__device__ __forceinline__ LineCoord line_coord(const LineGeo& geo, int64_t base, int w, int g,
-                                                int j, int tpl) {
+// Coordinates of line (w, g) of tile t.  y and z lines take them from the tile's
+// place among the TA x TB tiles of axis_geo; x lines divide their row number by
+// ny when asked (row_yz), since most passes need no coordinates.
+__device__ __forceinline__ LineCoord line_coord(const LineGeo& geo, int64_t t, int w, int g, int j,
+                                                int tpl) {
   LineCoord c;
-  c.idx0 = base + w + g * geo.gs + (int64_t)j * geo.ps;
+  const int64_t ta = t % geo.TA, tb = t / geo.TA;
+  c.idx0 = ta * geo.sa + tb * geo.sb + w + g * geo.gs + (int64_t)j * geo.ps;
   c.step = (int64_t)tpl * geo.ps;
-  c.x = c.y = c.z = 0;
-  if (geo.axis >= 0) {
-    const int64_t nxy = (int64_t)geo.nx * geo.ny;
-    const int64_t z = c.idx0 / nxy;
-    const int64_t r = c.idx0 - z * nxy;
-    const int64_t y = r / geo.nx;
-    c.x = (int)(r - y * geo.nx);
-    c.y = (int)y;
-    c.z = (int)z;
-  }
+  c.x = (int)ta * geo.W + w;
+  c.y = c.z = j;
+  (geo.axis == 2 ? c.y : c.z) = (int)tb * geo.G + g;
   return c;
+}
+__device__ __forceinline__ void row_yz(const LineGeo& geo, LineCoord& c, int j) {
+  if (geo.axis != 0) return;
+  const int64_t row = c.idx0 / geo.nx;
+  c.z = (int)(row / geo.ny);
+  c.y = (int)(row - (int64_t)c.z * geo.ny);
+  c.x = j;
 }
 
 // Tile of the b-th CTA of a pass over n tiles, walked from the last one when
@@ -119,8 +123,19 @@ __device__ __forceinline__ C pro_load(const C* __restrict__ src, const C* __rest
   }
 }
 
-// One tile of a line pass: field `blk mod nf`, tile `blk / nf` of `geo`;
-// ORD is the radix order of the line FFT (RadixOrder).
+// Field and tile of the blk-th CTA of a pass over nf fields (LineGeo::run).
+struct LineSlot {
+  int field;
+  int64_t t;
+};
+__device__ __forceinline__ LineSlot line_slot(int run, int64_t blk, int nf) {
+  const int64_t r = blk >> run;  // run r of nf fields' runs
+  const int64_t grp = r / nf;
+  return {(int)(r - grp * nf), (grp << run) + (blk & ((1 << run) - 1))};
+}
+
+// One tile of a line pass (line_slot); ORD is the radix order of the line FFT
+// (RadixOrder).
 template <typename T, int L, int PRO, typename Fields, int ORD = RADIX16_FIRST>
 __device__ __forceinline__ void line_pass_tile(const LineGeo& geo, const Fields& f, int nf,
                                                const cx_t<T>* __restrict__ tw, T sg, T scale,
@@ -130,9 +145,9 @@ __device__ __forceinline__ void line_pass_tile(const LineGeo& geo, const Fields&
   using P = LinePlan<L>;
   constexpr int E = P::E, TPL = P::TPL;
 
-  const int field = (int)(blk % nf);
-  const int64_t t = blk / nf;
-  const int64_t base = (t % geo.TA) * geo.sa + (t / geo.TA) * geo.sb;
+  // the omega fields read the tile's three components again: no runs there
+  const auto [field, t] =
+      line_slot(PRO == PRO_CURL6 || PRO == PRO_OMEGA ? 0 : geo.run, blk, nf);
   const int W = geo.W;
   const int w = threadIdx.x & (W - 1);
   const int s = threadIdx.x >> wshift;
@@ -140,7 +155,7 @@ __device__ __forceinline__ void line_pass_tile(const LineGeo& geo, const Fields&
   const int g = s / TPL;
   const int RS = tile_stride(L, W, (int)sizeof(C));
   C* row = sm + (w + W * g) * RS;
-  const LineCoord lc = line_coord(geo, base, w, g, j, TPL);
+  LineCoord lc = line_coord(geo, t, w, g, j, TPL);
 
   C v[E];
   {
@@ -160,6 +175,7 @@ __device__ __forceinline__ void line_pass_tile(const LineGeo& geo, const Fields&
       d1 = reinterpret_cast<const C*>(f.in(4));
     }
     // wavenumbers of the line: two are fixed, the one along the axis varies
+    if constexpr (PRO == PRO_CURL6 || PRO == PRO_OMEGA) row_yz(geo, lc, j);
     const T kx0 = geo.kx_half ? (T)lc.x : (T)freq_i(lc.x, geo.nx),
             ky0 = (T)freq_i(lc.y, geo.ny),
             kz0 = (T)freq_i(lc.z, geo.nz);
@@ -183,9 +199,9 @@ __device__ __forceinline__ void line_pass_tile(const LineGeo& geo, const Fields&
     // with this tile's loads in flight, the tile pf launches ahead into L2
     const int64_t bp = blk + geo.pf;
     if (geo.pf != 0 && bp >= 0 && bp < geo.TA * geo.TB * nf) {
-      const int64_t tp = bp / nf;
-      prefetch_lines<L>(reinterpret_cast<const char*>(f.in((int)(bp % nf))),
-                        (tp % geo.TA) * geo.sa + (tp / geo.TA) * geo.sb, W, geo.G, geo.gs,
+      const LineSlot p = line_slot(geo.run, bp, nf);
+      prefetch_lines<L>(reinterpret_cast<const char*>(f.in(p.field)),
+                        (p.t % geo.TA) * geo.sa + (p.t / geo.TA) * geo.sb, W, geo.G, geo.gs,
                         geo.ps, (int)sizeof(C), (int)blockDim.x);
     }
   }
@@ -194,6 +210,7 @@ __device__ __forceinline__ void line_pass_tile(const LineGeo& geo, const Fields&
   C* __restrict__ dst = reinterpret_cast<C*>(f.out(field));
   const bool do_scale = flags & PASS_SCALE;
   const bool do_zero = flags & PASS_ZERO_NYQUIST;
+  if (do_zero) row_yz(geo, lc, j);
   const bool line_on_plane = (geo.axis != 0 && !geo.kx_half && lc.x == (geo.nx >> 1)) ||
                              (geo.axis != 1 && lc.y == (geo.ny >> 1)) ||
                              (geo.axis != 2 && lc.z == (geo.nz >> 1));
@@ -209,10 +226,9 @@ __device__ __forceinline__ void line_pass_tile(const LineGeo& geo, const Fields&
 }
 
 // One tile of a plain-load line pass (PRO_LOAD) whose input is already in
-// shared memory (`stage`, put there by the TMA as one box of field `blk mod
-// nf`): position p of line (w, g) at (g L + p) W + w for y lines (the box's
-// [z][y][x] order, groups along z) and at (p G + g) W + w for z lines (groups
-// along y).  The arithmetic and the epilogue are line_pass_tile's on the same
+// shared memory (`stage`, put there by the TMA as one box): position p of line
+// (w, g) at (g L + p) W + w for y lines (the box's [z][y][x] order, groups along
+// z) and at (p G + g) W + w for z lines (groups along y).  The arithmetic and the epilogue are line_pass_tile's on the same
 // values, so both give the same bits.  after_reads() is called by every
 // thread once the tile's reads of the stage are issued (the CTA may then
 // refill it).
@@ -225,9 +241,7 @@ __device__ __forceinline__ void line_pass_tile_staged(const LineGeo& geo, const 
   using C = cx_t<T>;
   using P = LinePlan<L>;
   constexpr int E = P::E, TPL = P::TPL;
-  const int field = (int)(blk % nf);
-  const int64_t t = blk / nf;
-  const int64_t base = (t % geo.TA) * geo.sa + (t / geo.TA) * geo.sb;
+  const auto [field, t] = line_slot(geo.run, blk, nf);
   const int W = geo.W, G = geo.G;
   const int w = threadIdx.x & (W - 1);
   const int s = threadIdx.x >> wshift;
@@ -235,7 +249,7 @@ __device__ __forceinline__ void line_pass_tile_staged(const LineGeo& geo, const 
   const int g = s / TPL;
   const int RS = tile_stride(L, W, (int)sizeof(C));
   C* row = sm + (w + W * g) * RS;
-  const LineCoord lc = line_coord(geo, base, w, g, j, TPL);
+  LineCoord lc = line_coord(geo, t, w, g, j, TPL);
   // x and y lines: [g][p][w] (x lines have W = 1); z lines: [p][g][w]
   const bool ylines = geo.axis != 2;
   const int q0 = ylines ? (g * L + j) * W + w : (j * G + g) * W + w;
@@ -249,6 +263,7 @@ __device__ __forceinline__ void line_pass_tile_staged(const LineGeo& geo, const 
   C* __restrict__ dst = reinterpret_cast<C*>(f.out(field));
   const bool do_scale = flags & PASS_SCALE;
   const bool do_zero = flags & PASS_ZERO_NYQUIST;
+  if (do_zero) row_yz(geo, lc, j);
   const bool line_on_plane = (geo.axis != 0 && !geo.kx_half && lc.x == (geo.nx >> 1)) ||
                              (geo.axis != 1 && lc.y == (geo.ny >> 1)) ||
                              (geo.axis != 2 && lc.z == (geo.nz >> 1));
@@ -279,7 +294,6 @@ __device__ __forceinline__ void curl_zpass_tile(const LineGeo& geo, const Fields
   constexpr int E = P::E, TPL = P::TPL;
   const int W = geo.W, G = geo.G, lines = W * G;
   const int RS = tile_stride(L, W, (int)sizeof(C));
-  const int64_t base = (blk % geo.TA) * geo.sa + (blk / geo.TA) * geo.sb;
   prefetch_curl_tile<L, C>(geo, f, blk + geo.pf);
   const int w = threadIdx.x & (W - 1);
   const int s = threadIdx.x >> wshift;
@@ -289,7 +303,7 @@ __device__ __forceinline__ void curl_zpass_tile(const LineGeo& geo, const Fields
   const int li = w + W * g;
   C* rowV = sm + (d * lines + li) * RS;
   C* rowW = sm + ((3 + d) * lines + li) * RS;
-  const LineCoord lc = line_coord(geo, base, w, g, j, TPL);
+  const LineCoord lc = line_coord(geo, blk, w, g, j, TPL);
 
   C v[E];
   {
@@ -357,7 +371,6 @@ __device__ __forceinline__ void curl_zpass_tile_reload(const LineGeo& geo, const
   constexpr int E = P::E, TPL = P::TPL;
   const int W = geo.W, G = geo.G, lines = W * G;
   const int RS = tile_stride(L, W, (int)sizeof(C));
-  const int64_t base = (blk % geo.TA) * geo.sa + (blk / geo.TA) * geo.sb;
   prefetch_curl_tile<L, C>(geo, f, blk + geo.pf);
   const int w = threadIdx.x & (W - 1);
   const int s = threadIdx.x >> wshift;
@@ -365,7 +378,7 @@ __device__ __forceinline__ void curl_zpass_tile_reload(const LineGeo& geo, const
   const int s2 = s / TPL;
   const int g = s2 % G, d = s2 / G;  // line (w, g) of component d
   C* row = sm + (d * lines + w + W * g) * RS;
-  const LineCoord lc = line_coord(geo, base, w, g, j, TPL);
+  const LineCoord lc = line_coord(geo, blk, w, g, j, TPL);
   const C* __restrict__ v0 = reinterpret_cast<const C*>(f.in(0));
   const C* __restrict__ v1 = reinterpret_cast<const C*>(f.in(1));
   const C* __restrict__ v2 = reinterpret_cast<const C*>(f.in(2));
@@ -428,14 +441,13 @@ __device__ __forceinline__ void curl_zpass_tile_staged(const LineGeo& geo, const
   constexpr int E = P::E, TPL = P::TPL;
   const int W = geo.W, G = geo.G, lines = W * G;
   const int RS = tile_stride(L, W, (int)sizeof(C));
-  const int64_t base = (blk % geo.TA) * geo.sa + (blk / geo.TA) * geo.sb;
   const int w = threadIdx.x & (W - 1);
   const int s = threadIdx.x >> wshift;
   const int j = s & (TPL - 1);
   const int s2 = s / TPL;
   const int g = s2 % G, d = s2 / G;  // line (w, g) of component d
   C* row = sm + (d * lines + w + W * g) * RS;
-  const LineCoord lc = line_coord(geo, base, w, g, j, TPL);
+  const LineCoord lc = line_coord(geo, blk, w, g, j, TPL);
   const int q0 = j * lines + g * W + w, qs = TPL * lines, comp = L * lines;
   C v[E];
   {
