@@ -174,6 +174,20 @@ static int dispatch_pass(const LineGeo& geo, const FieldPtrs& f, int sign, int f
   }
 }
 
+template <typename T>
+static int dispatch_rows(const LineGeo& geo, const FieldPtrs& f, int sign, int flags, double scale,
+                         cudaStream_t stream) {
+  switch (geo.L) {
+    case 8: return launch_pass<T, 8, PRO_ROWS>(geo, f, sign, flags, scale, stream);
+    case 16: return launch_pass<T, 16, PRO_ROWS>(geo, f, sign, flags, scale, stream);
+    case 32: return launch_pass<T, 32, PRO_ROWS>(geo, f, sign, flags, scale, stream);
+    default:
+      if constexpr (sizeof(T) == 4)
+        return launch_pass<T, 64, PRO_ROWS>(geo, f, sign, flags, scale, stream);
+      return ERR_UNSUPPORTED;
+  }
+}
+
 int run_line_pass(const LineGeo& geo, const FieldPtrs& f, int sign, int flags, double scale,
                   int prec, cudaStream_t stream, int prologue) {
   if (f.n < 1 || f.n > kMaxFields) {
@@ -218,6 +232,12 @@ int run_line_pass(const LineGeo& geo, const FieldPtrs& f, int sign, int flags, d
       return dispatch_pass<double, PRO_IKAXIS>(geo, f, sign, flags, scale, stream);
     return dispatch_pass<float, PRO_IKAXIS>(geo, f, sign, flags, scale, stream);
   }
+  // short rows through shared memory: from 8 elements to 512 bytes (the figures
+  // are at line_pass_tile)
+  if (geo.axis == 0 && (geo.ord == RADIX16_FIRST || geo.L < 64) && geo.L >= 8 &&
+      geo.L <= (prec == PREC_C128 ? 32 : 64))
+    return prec == PREC_C128 ? dispatch_rows<double>(geo, f, sign, flags, scale, stream)
+                             : dispatch_rows<float>(geo, f, sign, flags, scale, stream);
   if (prec == PREC_C128) return dispatch_pass<double, PRO_LOAD>(geo, f, sign, flags, scale, stream);
   return dispatch_pass<float, PRO_LOAD>(geo, f, sign, flags, scale, stream);
 }

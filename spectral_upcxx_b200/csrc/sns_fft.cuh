@@ -61,6 +61,7 @@ enum PassPrologue : int {
                    // in[3..4] = the z-inverted i kz Vx, i kz Vy; fields 0..2
                    // read V, fields 3..5 form omega = i k x V from them
                    // (i ky Vz - dzVy, dzVx - i kx Vz, i kx Vy - i ky Vx)
+  PRO_ROWS = 5,    // PRO_LOAD on short x lines, through shared memory
 };
 
 // Geometry of a batch of lines: element p of line (w, g) of tile t sits at
