@@ -42,9 +42,9 @@ FALLBACK_HBM_GBS = 6650.0
 # (N^3 elements): the bytes it must read and write once.
 PASSES = {
     5: (["K1 z-inverse+curl", "K2 y-inverse x6", "K3 x-inv+cross+x-fwd", "K4 y-forward x3",
-         "K5 z-forward+update"], [3 + 6, 6 + 6, 6 + 3, 3 + 3, 9 + 6]),
+         "K5 z-forward+update"], [3 + 6, 6 + 6, 6 + 3, 3 + 3, 9 + 3]),
     3: (["K1 z-inverse+curl", "K234 xy %s (y-inv x6, x cross, y-fwd x3)",
-         "K5 z-forward+update"], [3 + 6, 6 + 3, 9 + 6]),
+         "K5 z-forward+update"], [3 + 6, 6 + 3, 9 + 3]),
 }
 
 
@@ -52,9 +52,9 @@ def pass_names(npasses, plan):
     """Names of the timed passes; the xy phase is named by the plan's mode.
     A plan whose update pass carries the next step's K1 ("(+K1") runs K1 in
     its first step only: the update pass then also writes the six z-inverted
-    fields (9 + 6 + 6) and K1's steady-state share is empty."""
+    fields (9 + 3 + 6) and K1's steady-state share is empty."""
     names, fields = PASSES[npasses]
-    mode = "cluster" if "xy=cluster" in plan else "dataflow" if "xy=dataflow" in plan else "slabs"
+    mode = next((m for m in ("cluster", "dataflow", "plane") if f"xy={m}" in plan), "slabs")
     names = [nm % mode if "%s" in nm else nm for nm in names]
     if "(+K1" in plan:
         names = names[:-1] + ["K5+K1 z-forward+update+z-inverse+curl"]
@@ -70,7 +70,7 @@ NCU_TRAFFIC = {
     ("ns256_fp32", "K2 y-inverse x6"): (810 + 749) * 1e6,
     ("ns256_fp32", "K3 x-inv+cross+x-fwd"): (805 + 359) * 1e6,
     ("ns256_fp32", "K4 y-forward x3"): (403 + 341) * 1e6,
-    ("ns256_fp32", "K5 z-forward+update"): (1208 + 752) * 1e6,
+    ("ns256_fp32", "K5 z-forward+update"): (1208 + 372) * 1e6,
 }
 
 WORKLOADS = {

@@ -55,6 +55,8 @@ int sns_version(void);
  * a later sns_malloc may hand it out again for work on the same stream. */
 int sns_malloc(void** ptr, size_t bytes);
 int sns_free(void* ptr);
+/* Give the pool's free blocks (and the free scratch of the tracer moves) back to
+ * the device. */
 int sns_pool_trim(void);
 int sns_memcpy_h2d(void* dst, const void* src, size_t bytes, void* stream);
 int sns_memcpy_d2h(void* dst, const void* src, size_t bytes, void* stream);
@@ -202,8 +204,8 @@ int sns_ns_set_state(sns_ns* handle, const void* const V1[3], const void* const 
 /* Advance nsteps AB2 / projection / Crank-Nicolson steps (ns.cpp:167-217),
  * queued on the stepper's stream without host synchronisation.  After the
  * first step the step's launches are captured once as a CUDA graph (on a
- * private stream) and replayed; environment SNS_GRAPH=0 at creation keeps
- * direct launches.  Changing the closure drops the captured graph. */
+ * private stream) and replayed -- for small boxes eight steps at a time, while as
+ * many are left; environment SNS_GRAPH=0 at creation keeps direct launches.  Changing the closure drops the captured graph. */
 int sns_ns_step(sns_ns* handle, int nsteps);
 /* Copy out V1, omega1 = curl V1 and cross0 (any pointer may be NULL). */
 int sns_ns_get_state(sns_ns* handle, void* const V1[3], void* const omega1[3],
@@ -247,8 +249,9 @@ int sns_ns_tune(sns_ns* handle);
 /* The stepper's plan as text (no reference counterpart; the reference's
  * planning is FFTW_MEASURE per line plan, src/FFT1D.cpp:18-22): the pass
  * structure and tile shapes chosen for this box, e.g.
- * "passes=5 xy=separate k1=8x1(tma1) y=W16/T256/16-first zW=16 xG=4(tma) pf=0 tuned".  Writes at most len bytes
- * (NUL-terminated) to buf; returns the full length. */
+ * "passes=5 xy=separate k1=8x1(tma1) y=W16/T128/16-first(tma1) zW=16(pfs) xG=2 pf=0 tuned"
+ * (xy=plane: the xy phase with one CTA per plane, K1 carried in the update pass).
+ * Writes at most len bytes (NUL-terminated) to buf; returns the full length. */
 int sns_ns_describe(sns_ns* handle, char* buf, int len);
 /* Per-pass timing (no reference counterpart; the reference times phases with
  * CH_Timer, src/Scalar.cpp:421-617).  While enabled, every step records CUDA

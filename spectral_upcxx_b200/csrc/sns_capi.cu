@@ -146,7 +146,7 @@ bool nonnull(const void* p, const char* what) {
 // rides on the last pass before the x lines, and the x lines of all six
 // fields, the product and its x transform are one pass (K3 of the step; on
 // planes that fit a CTA the y lines too): 45 field passes instead of 75.
-// B200, 128^3 complex128: 0.477 -> 0.320 ms.
+// B200, 128^3 complex128: 0.477 -> 0.294 ms.
 int vector_cross(const void* const a[3], const void* const b[3], void* const out[3], Dims d,
                  int prec, void* const scratch[6], cudaStream_t s, const void* const* tw_axes) {
   const double N = (double)d.n();
@@ -731,9 +731,9 @@ int sns::ns_create(sns_ns** handle, int64_t nx, int64_t ny, int64_t nz, double n
   for (int i = 0; i < 12 && rc == OK; i++) rc = pool_malloc(all[i], bytes);
   // SNS_K1_LINES=1: K1 as a line pass of V and i kz V into five more work
   // fields, the curl formed in K2 (and a candidate of the tuner).  Measured on
-  // B200 at 256^3 complex64 it loses: the z line pass runs at 3.1 TB/s like
-  // the fused K1 tile (0.351 vs 0.394 ms) while the omega prologue's extra
-  // loads slow K2 from 0.297 to 0.522 ms.
+  // B200 at 256^3 complex64 it loses: the z line pass takes about as long as
+  // the fused K1 tile (0.259 vs 0.271 ms) while the omega prologue's extra
+  // loads slow K2 from 0.282 to 0.504 ms.
   const char* kl = getenv("SNS_K1_LINES");
   if (rc == OK && kl && kl[0] == '1') {
     for (int i = 0; i < kNSLineWork && rc == OK; i++) rc = pool_malloc(&h->W[i], bytes);

@@ -98,8 +98,9 @@ struct LineGeo {
 // Run of a pass over several fields: up to 64 tiles.  The CTAs of a wave then
 // stream through few fields at a time, and a pass still ends on the same planes of
 // all its fields, where the next one starts (`rev`).  y-inverse of six 256^3 fields
-// on B200, complex64 staged / complex128: runs of 1 tile 0.287 / 0.521 ms, 64 tiles
-// 0.277 / 0.516, whole fields 0.275 / 0.512 with 2 to 3 us lost in the x pass.
+// on B200, complex64 staged / complex128: runs of 1 tile 0.301 / 0.501 ms, 64 tiles
+// 0.282 / 0.499; whole fields gain 2 to 4 us more there and lose 2 to 3 in the x
+// pass that follows.
 inline int field_run(int64_t tiles) {
   int run = 0;
   while (run < 6 && tiles % ((int64_t)2 << run) == 0) run++;

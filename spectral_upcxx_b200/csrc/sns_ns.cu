@@ -288,8 +288,8 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   // move a third of their HBM bytes but measured slower on B200, the passes
   // being bound by latency and issue rather than bytes: SNS_XYC=1 selects one
   // thread-block-cluster pass over each plane (sns_xyc.cu; nx = ny = 128, or
-  // 256 in complex64; 1.28 vs 0.73 ms at 256^3), SNS_XY_PASSES=1 the
-  // persistent dataflow launch through L2 (sns_xy.cu; 1.09 vs 0.79 ms).
+  // 256 in complex64; 1.28 vs 0.69 ms at 256^3), SNS_XY_PASSES=1 the
+  // persistent dataflow launch through L2 (sns_xy.cu; 1.13 vs 0.69 ms).
   // K1 walks its tiles back from where K5 ended (both follow the xy plane),
   // K3 back from where K2 ended (both follow z).  B200, whole complex64 step:
   // 0.5 to 1 % at 256^3, 3.5 % at 128^3.
@@ -864,9 +864,9 @@ int ns_tune_plan(NSPlan& pl, void* const V[3], void* const C0[3], void* const U[
   }
   // K5 with the next step's K1 carried in it (tile widths), against the
   // plan so far, over the whole step: it trades K1's pass for a heavier K5.
-  // Measured slower in steady state on B200 at 256^3 (whole step 1.53 against
-  // 1.45 ms, and 0.78 against 0.71 ms for K5 + K1 in a long run), so it is
-  // only tried on request (SNS_TUNE_CARRY=1)
+  // Measured slower in steady state on B200 at 256^3 (whole step 1.37 to 1.44
+  // against 1.30 ms; complex128 2.74 to 2.90 against 2.57), so it is only tried
+  // on request (SNS_TUNE_CARRY=1)
   const char* etc = getenv("SNS_TUNE_CARRY");
   if (rc == OK && !pl.k1_lines && !getenv("SNS_CARRY") && etc && etc[0] == '1') {
     c.clear();

@@ -38,8 +38,8 @@
 // 39 us whether one cluster or seven run: y-inverse of the six fields with
 // the stores to the row owners 15 us, x-inverse 7.2, x-forward 3.7, y-forward
 // 3.5, product exchange 2.9, cross product 1.4, the four cluster barriers
-// 3.6 us.  The phase takes 1.28 ms against 0.73 ms for the three separate
-// passes (0.158 against 0.109 ms at 128^3), so the stepper uses the separate
+// 3.6 us.  The phase takes 1.28 ms against 0.69 ms for the three separate
+// passes (0.163 against 0.097 ms at 128^3), so the stepper uses the separate
 // passes and this pass is opt-in (SNS_XYC=1).
 #include <stdlib.h>
 
