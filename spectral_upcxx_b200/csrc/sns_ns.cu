@@ -333,8 +333,8 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   {
     // K1 over TMA-staged tiles, one stage by default (SNS_K1_TMA = 0: off,
     // 2: two stages); an explicit SNS_K1_RELOAD=1 or SNS_K1_SPLIT=1 keeps
-    // that form.  Measured on B200 at 256^3: complex64 0.28 ms against 0.37
-    // (reload tile), complex128 0.58 against 0.79 (split).
+    // that form.  Measured on B200 at 256^3: complex64 0.27 ms against 0.37
+    // (reload tile), complex128 0.50 against 0.92 (reload; 0.79 split, before).
     const char* e = getenv("SNS_K1_TMA");
     const char* es = getenv("SNS_K1_SPLIT");
     const int v = e ? atoi(e) : ((pl.k1_reload || (es && es[0] == '1')) ? 0 : 1);

@@ -102,6 +102,15 @@ int ns_update_carry(const NSPlan& pl, const UpdateArgs& a, cudaStream_t s);
 
 #ifdef SNS_NS_PASSES
 
+// Largest CTA of the z passes.  Their thread counts are 3 or 9 times a power of
+// two, so complex128 ones of up to 512 threads have at most 384, and compiled for
+// that they have 168 registers instead of 128: a 384-thread CTA has the SM to
+// itself either way, and K1's 100 bytes of spills a thread go (B200, 256^3:
+// TMA-staged K1 0.542 -> 0.501 ms, K5 0.706 -> 0.685; 128^3 74.4 -> 68.5 and 95.5
+// -> 93.3 us).
+template <typename T>
+constexpr int kZThreads = sizeof(T) == 8 ? 384 : MaxThreads<T>::value;
+
 // ---------------------------------------------------------------------------
 // K3: x lines -- inverse 6 fields, cross product, forward 3 fields.
 template <typename T, int L>
@@ -245,7 +254,7 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 // that path: the first tile's wait also waits that long on a barrier that
 // nothing arrives at.
 template <typename T, int L, int S>
-__global__ void __launch_bounds__(MaxThreads<T>::value)
+__global__ void __launch_bounds__(kZThreads<T>)
     k_zcurl_tma(const __grid_constant__ CUtensorMap m0, const __grid_constant__ CUtensorMap m1,
                 const __grid_constant__ CUtensorMap m2, const LineGeo geo, const FieldPtrs f,
                 const cx_t<T>* __restrict__ tw, int wshift, int* err, long long stall_cycles) {
@@ -340,7 +349,7 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 // K5: z lines -- forward 3 fields + Nyquist zeroing, then the AB2 /
 // projection / CN update per mode.
 template <typename T, int L, bool SGS>
-__global__ void __launch_bounds__(MaxThreads<T>::value)
+__global__ void __launch_bounds__(kZThreads<T>)
     k_zfwd_update(const UpdateArgs a, const cx_t<T>* __restrict__ tw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[4][32];
@@ -353,7 +362,7 @@ __global__ void __launch_bounds__(MaxThreads<T>::value)
 // K5 with the next step's K1 carried in it (zfwd_update_curl_tile): the
 // update, then the z-inverse of the new V and of i k x V into a.Uo.
 template <typename T, int L, bool RELOAD, int EM = 16>
-__global__ void __launch_bounds__(MaxThreads<T>::value)
+__global__ void __launch_bounds__(kZThreads<T>)
     k_zfwd_update_curl(const UpdateArgs a, const cx_t<T>* __restrict__ tw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[4][32];
