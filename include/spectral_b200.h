@@ -205,7 +205,12 @@ int sns_ns_set_state(sns_ns* handle, const void* const V1[3], const void* const 
  * queued on the stepper's stream without host synchronisation.  After the
  * first step the step's launches are captured once as a CUDA graph (on a
  * private stream) and replayed -- for small boxes eight steps at a time, while as
- * many are left; environment SNS_GRAPH=0 at creation keeps direct launches.  Changing the closure drops the captured graph. */
+ * many are left; environment SNS_GRAPH=0 at creation keeps direct launches.
+ * Changing the closure drops the captured graph.  Under a capture of the caller's
+ * the launches themselves are captured; replays advance the state as direct calls
+ * do and may be mixed with them.  The first captured call that reads or writes
+ * the state waits for the steps queued before, and from then on each call of
+ * sns_ns_step ends with one z transform of the history. */
 int sns_ns_step(sns_ns* handle, int nsteps);
 /* Copy out V1, omega1 = curl V1 and cross0 (any pointer may be NULL). */
 int sns_ns_get_state(sns_ns* handle, void* const V1[3], void* const omega1[3],
@@ -380,7 +385,7 @@ int sns_ens_set_state(sns_ens* handle, int box, const void* const V1[3],
 int sns_ens_get_state(sns_ens* handle, int box, void* const V1[3], void* const omega1[3],
                       void* const cross0[3]);
 /* Advance every box nsteps steps (mode: SNS_ENS_GRAPH, _EAGER, _SEQUENTIAL),
- * queued on the ensemble's stream. */
+ * queued on the ensemble's stream; captures of the caller's as for sns_ns_step. */
 int sns_ens_step(sns_ens* handle, int nsteps, int mode);
 /* Diagnostics of every box after the last step, 4 doubles per box in the
  * order of sns_ns_stats (div_avg, energy, enstrophy, max_div).  Synchronises. */

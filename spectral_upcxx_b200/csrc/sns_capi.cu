@@ -305,6 +305,11 @@ struct sns_ns {
   bool carried = false;
   // where the history cross0 is (HIST_*)
   int hist = HIST_FOURIER;
+  // The caller captures steps into graphs of its own.  A replay finds the fields
+  // where the captured calls had them, so from the first such call on every call
+  // leaves the history in its Fourier form in C0 (settle, settled).
+  bool canonical = false;
+  cudaEvent_t last = nullptr;  // after the steps queued so far
   // eddy-viscosity closure (none by default) and its six extra work fields
   Closure cl;
   void* U2[6] = {};
@@ -339,13 +344,44 @@ void drop_graph(sns_ns* h) {
 }
 
 // The history into its Fourier form in C0, for what reads it there.
-int hist_to_fourier(sns_ns* h) {
+int hist_to_fourier(sns_ns* h, cudaStream_t s) {
   if (h->hist == HIST_FOURIER) return OK;
-  const int rc = ns_hist_fourier(h->pl, h->hist == HIST_Z_U ? h->U : h->C0, h->C0, 3, h->s);
+  const int rc = ns_hist_fourier(h->pl, h->hist == HIST_Z_U ? h->U : h->C0, h->C0, 3, s);
   if (rc) return rc;
   h->hist = HIST_FOURIER;
   h->carried = false;  // U[0..2] or C0 no longer is what a carried K1 wrote
   return OK;
+}
+
+// Before a call that reads or writes the fields: whether its stream is being
+// captured.  At the first such call the history goes to C0 outside the capture,
+// after the work queued before it (the replays are later work).
+int settle(sns_ns* h, bool* captured) {
+  *captured = stream_captured(h->s);
+  if (!*captured || h->canonical) return OK;
+  if (h->hist != HIST_FOURIER) {
+    const RelaxedCapture relaxed;
+    int rc = OK;
+    if (!h->cap)
+      rc = cuda_status(cudaStreamCreateWithFlags(&h->cap, cudaStreamNonBlocking), "sns_ns capture");
+    if (!rc) rc = cuda_status(cudaStreamWaitEvent(h->cap, h->last, 0), "sns_ns capture");
+    if (!rc) rc = hist_to_fourier(h, h->cap);
+    if (!rc) rc = cuda_status(cudaStreamSynchronize(h->cap), "sns_ns capture");
+    if (rc) return rc;
+  }
+  h->canonical = true;
+  return OK;
+}
+
+// After steps.
+int settled(sns_ns* h) {
+  if (h->canonical) return hist_to_fourier(h, h->s);
+  if (h->hist == HIST_FOURIER) return OK;
+  if (!h->last)
+    if (int rc = cuda_status(cudaEventCreateWithFlags(&h->last, cudaEventDisableTiming),
+                             "sns_ns_step"))
+      return rc;
+  return cuda_status(cudaEventRecord(h->last, h->s), "sns_ns_step");
 }
 
 // One step (plain or closure) queued on `s`.
@@ -356,7 +392,7 @@ int step_on(sns_ns* h, cudaStream_t s, cudaEvent_t* ev) {
       U[i] = h->U[i];
       U[6 + i] = h->U2[i];
     }
-    if (int rc = hist_to_fourier(h)) return rc;
+    if (int rc = hist_to_fourier(h, s)) return rc;
     h->carried = false;  // the closure step uses U as work space
     return les_step_once(h->pl, h->V, h->C0, U, h->stats_part, h->nu, h->dt, h->cl, s);
   }
@@ -787,6 +823,7 @@ int sns_ns_destroy(sns_ns* h) {
   drop_graph(h);
   h->carried = false;
   if (h->cap) cudaStreamDestroy(h->cap);
+  if (h->last) cudaEventDestroy(h->last);
   delete h;
   return OK;
 }
@@ -795,6 +832,8 @@ int sns_ns_set_state(sns_ns* h, const void* const V1[3], const void* const cross
   if (!nonnull(h, "sns_ns_set_state") || !vec_ok(V1, "sns_ns_set_state") ||
       !vec_ok(cross0, "sns_ns_set_state"))
     return ERR_ARG;
+  bool captured;
+  if (int rc = settle(h, &captured)) return rc;
   if (h->pl.real) {
     int rc = convert_half(h->V, V1, h->pl.nx_phys, h->pl.ny, h->pl.nz, h->pl.prec, +1, h->s);
     if (!rc) rc = convert_half(h->C0, cross0, h->pl.nx_phys, h->pl.ny, h->pl.nz, h->pl.prec, +1,
@@ -820,7 +859,9 @@ int sns_ns_bootstrap(sns_ns* h, const void* const V0[3], const void* const omega
   if (!nonnull(h, "sns_ns_bootstrap") || !vec_ok(V0, "sns_ns_bootstrap") ||
       !vec_ok(omega0, "sns_ns_bootstrap"))
     return ERR_ARG;
-  int rc;
+  bool captured;
+  int rc = settle(h, &captured);
+  if (rc) return rc;
   if (h->pl.real) {
     // bootstrap on full fields (pooled temporaries), then keep the half spectrum
     const Dims d{h->pl.nx_phys, h->pl.ny, h->pl.nz};
@@ -855,6 +896,8 @@ int sns_ns_step(sns_ns* h, int nsteps) {
     set_error("sns_ns_step: negative step count");
     return ERR_ARG;
   }
+  bool captured;
+  if (int rc = settle(h, &captured)) return rc;
   if (!h->profiling) {
     // (a closure step's launches overlap their neighbours' edges, which measured
     // slower across steps: 72 -> 79 us a 64^3 step)
@@ -865,7 +908,9 @@ int sns_ns_step(sns_ns* h, int nsteps) {
       // make it there first if the state was set since
       // (a Fourier history serves the one step after it was set, launched directly)
       const bool plain = h->cl.model == CLOSURE_NONE;
-      const bool replay = h->use_graph && h->eager_done && !(plain && h->hist == HIST_FOURIER);
+      // (a caller's capture takes the launches themselves)
+      const bool replay = h->use_graph && h->eager_done && !captured &&
+                          !(plain && h->hist == HIST_FOURIER);
       if (replay && plain && h->pl.carry && !h->carried) {
         if ((rc = ns_k1_once(h->pl, h->V, h->C0, h->U, h->hist, h->sync_words, h->s))) return rc;
         h->carried = true;
@@ -890,7 +935,7 @@ int sns_ns_step(sns_ns* h, int nsteps) {
       if (rc) return rc;
       h->stepped = true;
     }
-    return OK;
+    return settled(h);
   }
   if (h->cl.model != CLOSURE_NONE) {
     set_error("sns_ns_step: per-pass profiling covers the plain step only");
@@ -914,7 +959,7 @@ int sns_ns_step(sns_ns* h, int nsteps) {
     if (ev) h->recorded++;
     h->stepped = true;
   }
-  return OK;
+  return settled(h);
 }
 
 int sns_ns_profile(sns_ns* h, int enable) {
@@ -949,6 +994,8 @@ int sns_ns_pass_times(sns_ns* h, double* total_ms, int* launches, int max) {
 
 int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* const cross0[3]) {
   if (!nonnull(h, "sns_ns_get_state")) return ERR_ARG;
+  bool captured;
+  if (int rc = settle(h, &captured)) return rc;
   if (h->pl.real) {
     // full spectra rebuilt by Hermitian symmetry
     const Dims d{h->pl.nx_phys, h->pl.ny, h->pl.nz};
@@ -997,7 +1044,7 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
   // a destination that only a byte copy can write
   for (int i = 0; i < 3 && cross0; i++)
     if (reinterpret_cast<uintptr_t>(cross0[i]) % esize(h->pl.prec))
-      if ((rc = hist_to_fourier(h))) return rc;
+      if ((rc = hist_to_fourier(h, h->s))) return rc;
   // V1 and its curl from one read of V where both are wanted
   bool both = omega1 && V1 && V1[0] && V1[1] && V1[2];
   for (int i = 0; i < 3 && both; i++)
@@ -1233,7 +1280,9 @@ int sns_ns_set_closure(sns_ns* h, int model, double cs_delta2, const void* mlp, 
     }
   }
   // the history with the cutoff it was made under
-  if (int rc = hist_to_fourier(h)) return rc;
+  bool captured;
+  if (int rc = settle(h, &captured)) return rc;
+  if (int rc = hist_to_fourier(h, h->s)) return rc;
   h->cl.model = model;
   h->cl.csd2 = cs_delta2;
   h->cl.mlp = mlp;

@@ -119,6 +119,22 @@ inline cudaError_t allow_max_dynamic_smem(K* kernel) {
 // Number of SMs of the current device (cached).
 int sm_count();
 
+// Whether work queued on s now goes into a graph that is being captured.
+inline bool stream_captured(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+// Calls that a capture on another stream of this thread would forbid.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 }  // namespace sns
 
 // Programmatic dependent launch.  A kernel started by launch_pdl inside a

@@ -275,6 +275,11 @@ struct sns_ens {
   int turn = 0;
   int* d_fourier = nullptr;   // per box (table order): its history is Fourier
   std::vector<char> pending;  // the same on the host
+  // the caller captures steps into graphs of its own: from the first such call on
+  // every call leaves all histories Fourier in C0, where a replay looks for them
+  // (settle, settled)
+  bool canonical = false;
+  cudaEvent_t last = nullptr;  // after the steps queued so far
   EnsClass* d_cls = nullptr;  // kEnsStages x nclass
   int64_t* d_parts_ens = nullptr;
   int64_t* d_parts_seq = nullptr;
@@ -481,6 +486,51 @@ int mark_fourier(sns_ens* e, int i) {
   return cuda_status(cudaMemsetAsync(e->d_fourier + i, 1, sizeof(int), e->s), "sns_ens_set_state");
 }
 
+// Every history Fourier in C0.
+int to_fourier(sns_ens* e, cudaStream_t s) {
+  const int nb = (int)e->boxes.size();
+  for (int i = 0; i < nb; i++) {
+    const BoxHost& b = e->boxes[i];
+    const size_t bytes = esize_of(e->prec) * (size_t)b.nx * b.ny * b.nz;
+    void* const* h = history(e, i);
+    void *src[3], *dst[3];
+    const void* from[3];
+    for (int d = 0; d < 3; d++) {
+      from[d] = src[d] = h[d];
+      dst[d] = b.C0[d];
+    }
+    int rc = OK;
+    if (!e->pending[i])
+      rc = ns_hist_fourier(e->classes[b.cls].seq, src, dst, 3, s);
+    else if (e->turn)
+      rc = op_copy_fields(from, dst, 3, bytes, s);
+    if (rc) return rc;
+  }
+  e->turn = 0;
+  e->pending.assign(nb, 1);
+  return cuda_status(cudaMemsetAsync(e->d_fourier, 1, sizeof(int) * nb, s), "sns_ens_step");
+}
+
+// Before a call that reads or writes the fields: whether its stream is being
+// captured.  At the first such call the histories go to C0 outside the capture,
+// after the work queued before it (the replays are later work).
+int settle(sns_ens* e, bool* captured) {
+  *captured = stream_captured(e->s);
+  if (!*captured || e->canonical) return OK;
+  const RelaxedCapture relaxed;
+  int rc = cuda_status(cudaStreamWaitEvent(e->cap, e->last, 0), "sns_ens capture");
+  if (!rc) rc = to_fourier(e, e->cap);
+  if (!rc) rc = cuda_status(cudaStreamSynchronize(e->cap), "sns_ens capture");
+  if (!rc) e->canonical = true;
+  return rc;
+}
+
+// After work on the fields.
+int settled(sns_ens* e) {
+  if (e->canonical) return to_fourier(e, e->s);
+  return cuda_status(cudaEventRecord(e->last, e->s), "sns_ens");
+}
+
 int launch_step(const sns_ens* e, cudaStream_t stream) {
   for (int s = 0; s < kEnsStages; s++) {
     int rc = launch_stage(e, s, stream);
@@ -587,6 +637,7 @@ void release(sns_ens* e) {
   pool_free(e->d_parts_seq);
   pool_free(e->d_stats);
   if (e->cap) cudaStreamDestroy(e->cap);
+  if (e->last) cudaEventDestroy(e->last);
 }
 
 bool box_ok(const sns_ens* e, int box, const char* what) {
@@ -763,6 +814,9 @@ int sns_ens_create(sns_ens** handle, int nboxes, const int64_t* dims, const doub
   }
   if (!rc)
     rc = cuda_status(cudaStreamCreateWithFlags(&e->cap, cudaStreamNonBlocking), "sns_ens_create");
+  if (!rc)
+    rc = cuda_status(cudaEventCreateWithFlags(&e->last, cudaEventDisableTiming), "sns_ens_create");
+  if (!rc) rc = cuda_status(cudaEventRecord(e->last, e->s), "sns_ens_create");
   if (rc) {
     release(e);
     delete e;
@@ -786,6 +840,8 @@ int sns_ens_bootstrap(sns_ens* e, int box, const void* const V0[3], const void* 
   if (!box_ok(e, box, "sns_ens_bootstrap") || !vec3(V0, "sns_ens_bootstrap") ||
       !vec3(omega0, "sns_ens_bootstrap"))
     return ERR_ARG;
+  bool captured;
+  if (int rc = settle(e, &captured)) return rc;
   BoxHost& b = e->boxes[e->user_to_table[box]];
   const int i = e->user_to_table[box];
   const Dims d{(int)b.nx, (int)b.ny, (int)b.nz};
@@ -795,13 +851,15 @@ int sns_ens_bootstrap(sns_ens* e, int box, const void* const V0[3], const void* 
   if (!rc) rc = mark_fourier(e, i);
   if (rc) return rc;
   e->stepped = false;
-  return OK;
+  return settled(e);
 }
 
 int sns_ens_set_state(sns_ens* e, int box, const void* const V1[3], const void* const cross0[3]) {
   if (!box_ok(e, box, "sns_ens_set_state") || !vec3(V1, "sns_ens_set_state") ||
       !vec3(cross0, "sns_ens_set_state"))
     return ERR_ARG;
+  bool captured;
+  if (int rc = settle(e, &captured)) return rc;
   BoxHost& b = e->boxes[e->user_to_table[box]];
   const size_t bytes = esize_of(e->prec) * (size_t)b.nx * b.ny * b.nz;
   void* const* h = history(e, e->user_to_table[box]);
@@ -810,12 +868,14 @@ int sns_ens_set_state(sns_ens* e, int box, const void* const V1[3], const void* 
   if (int rc = op_copy_fields(src, dst, 6, bytes, e->s)) return rc;
   if (int rc = mark_fourier(e, e->user_to_table[box])) return rc;
   e->stepped = false;
-  return OK;
+  return settled(e);
 }
 
 int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1[3],
                       void* const cross0[3]) {
   if (!box_ok(e, box, "sns_ens_get_state")) return ERR_ARG;
+  bool captured;
+  if (int rc = settle(e, &captured)) return rc;
   BoxHost& b = e->boxes[e->user_to_table[box]];
   const Dims d{(int)b.nx, (int)b.ny, (int)b.nz};
   const size_t bytes = esize_of(e->prec) * (size_t)d.n();
@@ -879,7 +939,9 @@ int sns_ens_step(sns_ens* e, int nsteps, int mode) {
     set_error("sns_ens_step: bad step count or mode");
     return ERR_ARG;
   }
-  int rc = OK;
+  bool captured;
+  int rc = settle(e, &captured);
+  if (rc) return rc;
   // one ensemble step captured on the private stream, replayed on the caller's
   auto capture = [&]() -> int {
     if ((rc = cuda_status(cudaStreamBeginCapture(e->cap, cudaStreamCaptureModeThreadLocal),
@@ -902,10 +964,11 @@ int sns_ens_step(sns_ens* e, int nsteps, int mode) {
     return OK;
   };
   for (int t = 0; t < nsteps; t++) {
-    if (mode == SNS_ENS_GRAPH) {
+    if (mode == SNS_ENS_GRAPH && !captured) {
       if (!e->exec[e->turn] && (rc = capture())) return rc;
       rc = cuda_status(cudaGraphLaunch(e->exec[e->turn], e->s), "sns_ens_step(graph)");
-    } else if (mode == SNS_ENS_EAGER) {
+    } else if (mode != SNS_ENS_SEQUENTIAL) {
+      // (a caller's capture takes the launches themselves)
       rc = launch_step(e, e->s);
     } else {
       for (int i = 0; i < (int)e->boxes.size(); i++) {
@@ -926,7 +989,7 @@ int sns_ens_step(sns_ens* e, int nsteps, int mode) {
     e->stepped = true;
     e->last_mode = mode;
   }
-  return OK;
+  return settled(e);
 }
 
 int sns_ens_stats(sns_ens* e, double* out) {
@@ -995,6 +1058,7 @@ int sns_ens_stage_times(sns_ens* e, int nsteps, double* ms) {
       e->last_mode = SNS_ENS_EAGER;
     }
   }
+  if (!rc) rc = settled(e);
   if (!rc) rc = cuda_status(cudaStreamSynchronize(e->s), "sns_ens_stage_times");
   for (int s = 0; s < kEnsStages; s++) ms[s] = 0;
   for (int t = 0; t < nsteps && !rc; t++) {
