@@ -869,12 +869,13 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
       for (int e = 0; e < E; e++) row[pad_pos(j + TPL * e)] = v[e];
     }
   }
-  // The update.  W is a power of two that divides the thread count, so a thread
-  // keeps one (x, y) column of the tile and walks down z: kx, ky and the
-  // pointer step are loop constants (dividing the flat point index by the
-  // run-time W cost more instructions than the update's arithmetic).  The
-  // loads of the next point are issued before the current one is computed, the
-  // first ones before the rows' barrier.
+  // The update.  W is a power of two, so a thread keeps one (x, y) column of the
+  // tile and walks down z: kx, ky and the pointer step are loop constants
+  // (dividing the flat point index by the run-time W cost more instructions than
+  // the update's arithmetic).  Where W does not divide the thread count (a tile
+  // of one thread per line in two halves: 3 W / 2 threads) the last threads stay
+  // out, so that every column has its own.  The loads of the next point are issued
+  // before the current one is computed, the first ones before the rows' barrier.
   const T hK = (T)a.hK, nuhK = (T)a.nuhK;
   double s_div = 0, s_e = 0, s_w = 0;
   T m_div = 0;  // the FP64 maximum of FP32 values is one of them
@@ -894,6 +895,7 @@ __device__ __forceinline__ void zfwd_update_tile_from(const UpdateArgs& a,
   const double wgt = (a.kx_half && x > 0) ? 2.0 : 1.0;
   const bool cutoff = a.kc2 < 1e300;
   int z = threadIdx.x >> wsh;
+  if (z >= dz) z = L;
   const T len = (T)a.nz, step = (T)dz;
   T kz = (T)freq_i(z, a.nz);
   int64_t idx = xy + nxy * z;
