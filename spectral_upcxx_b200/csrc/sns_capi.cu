@@ -174,6 +174,14 @@ int vector_cross(const void* const a[3], const void* const b[3], void* const out
   for (int i = 0; i < 6; i++) {
     f.in[i] = const_cast<void*>(i < 3 ? a[i] : b[i - 3]);
     f.out[i] = scratch[i];
+    // an operand that only a byte copy can read
+    if (reinterpret_cast<uintptr_t>(f.in[i]) % esize(prec)) {
+      if ((rc = cuda_status(cudaMemcpyAsync(scratch[i], f.in[i], esize(prec) * d.n(),
+                                            cudaMemcpyDeviceToDevice, s),
+                            "cross copy")))
+        return rc;
+      f.in[i] = scratch[i];
+    }
   }
   if ((rc = fft_axis_pass(six, f, 2, +1, plane ? PASS_SCALE : 0, 1.0 / N, s))) return rc;
   if (plane) {

@@ -358,7 +358,10 @@ int fft_axis_pass(const FftShape& p, const FieldPtrs& f, int axis, int sign, int
   // inverse on B200: 0.293 ms against 0.303 in plain order).
   g.rev = (sign < 0) == (axis == 1);
   if (p.tw) g.tw = p.tw[axis];
-  const int S = p.tuned ? p.tc.tma[axis] : p.forced;
+  // (direct loads give the same bits and take fields that no TMA copy can start at)
+  int S = p.tuned ? p.tc.tma[axis] : p.forced;
+  for (int i = 0; i < f.n; i++)
+    if (reinterpret_cast<uintptr_t>(f.in[i]) % 16) S = 0;
   if (S && p.err && f.n <= 6 && line_tma_ok(g, p.prec, S))
     return run_line_pass_tma(g, f, sign, flags, scale, p.prec, stream, S, p.err);
   return run_line_pass(g, f, sign, flags, scale, p.prec, stream);
