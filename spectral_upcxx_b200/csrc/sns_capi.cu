@@ -27,6 +27,7 @@ const char* last_error() { return g_err.c_str(); }
 
 int cuda_status(cudaError_t e, const char* where) {
   if (e == cudaSuccess) return OK;
+  cudaGetLastError();  // reported here: not again by the check of the next launch
   set_error(std::string(where) + ": " + cudaGetErrorString(e));
   return e == cudaErrorMemoryAllocation ? ERR_ALLOC : ERR_CUDA;
 }
@@ -141,6 +142,12 @@ bool nonnull(const void* p, const char* what) {
   return true;
 }
 
+// A caller's field that kernels cannot take: off an element boundary, or of
+// another device.
+bool copy_only(const void* p, int prec) {
+  return reinterpret_cast<uintptr_t>(p) % esize(prec) || !on_this_device(p);
+}
+
 // Vector::cross on device fields (src/Vector.cpp:66-90), scratch = 6 fields.
 // The first pass reads the operands out of place (no copies of them), the 1/N
 // rides on the last pass before the x lines, and the x lines of all six
@@ -174,8 +181,8 @@ int vector_cross(const void* const a[3], const void* const b[3], void* const out
   for (int i = 0; i < 6; i++) {
     f.in[i] = const_cast<void*>(i < 3 ? a[i] : b[i - 3]);
     f.out[i] = scratch[i];
-    // an operand that only a byte copy can read
-    if (reinterpret_cast<uintptr_t>(f.in[i]) % esize(prec)) {
+    // an operand that only a copy can read
+    if (copy_only(f.in[i], prec)) {
       if ((rc = cuda_status(cudaMemcpyAsync(scratch[i], f.in[i], esize(prec) * d.n(),
                                             cudaMemcpyDeviceToDevice, s),
                             "cross copy")))
@@ -855,7 +862,7 @@ int sns_ns_set_state(sns_ns* h, const void* const V1[3], const void* const cross
   const size_t bytes = esize(h->pl.prec) * (size_t)h->pl.nx * h->pl.ny * h->pl.nz;
   const void* src[6] = {V1[0], V1[1], V1[2], cross0[0], cross0[1], cross0[2]};
   void* dst[6] = {h->V[0], h->V[1], h->V[2], h->C0[0], h->C0[1], h->C0[2]};
-  int rc = op_copy_fields(src, dst, 6, bytes, h->s);
+  int rc = op_copy_fields(src, dst, 6, bytes, src, h->s);
   if (rc) return rc;
   h->stepped = false;
   h->carried = false;
@@ -1049,14 +1056,14 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
   const Dims d{h->pl.nx, h->pl.ny, h->pl.nz};
   const size_t bytes = esize(h->pl.prec) * (size_t)d.n();
   int rc;
-  // a destination that only a byte copy can write
+  // a destination that only a copy can write
   for (int i = 0; i < 3 && cross0; i++)
-    if (reinterpret_cast<uintptr_t>(cross0[i]) % esize(h->pl.prec))
+    if (h->hist != HIST_FOURIER && cross0[i] && copy_only(cross0[i], h->pl.prec))
       if ((rc = hist_to_fourier(h, h->s))) return rc;
   // V1 and its curl from one read of V where both are wanted
   bool both = omega1 && V1 && V1[0] && V1[1] && V1[2];
   for (int i = 0; i < 3 && both; i++)
-    both = omega1[i] && reinterpret_cast<uintptr_t>(V1[i]) % esize(h->pl.prec) == 0;
+    both = omega1[i] && !copy_only(V1[i], h->pl.prec);
   if (both) {
     const void* v[3] = {h->V[0], h->V[1], h->V[2]};
     if ((rc = op_curl_copy(v, V1, omega1, d, h->pl.prec, h->s))) return rc;
@@ -1075,7 +1082,7 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
         dst[n++] = cross0[i];
       }
     }
-    if (n && (rc = op_copy_fields(src, dst, n, bytes, h->s))) return rc;
+    if (n && (rc = op_copy_fields(src, dst, n, bytes, dst, h->s))) return rc;
   }
   if (h->hist != HIST_FOURIER && cross0) {
     void *src[3], *dst[3];

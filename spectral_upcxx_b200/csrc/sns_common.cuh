@@ -119,6 +119,18 @@ inline cudaError_t allow_max_dynamic_smem(K* kernel) {
 // Number of SMs of the current device (cached).
 int sm_count();
 
+// Whether a kernel on the current device may read and write p.  Copies also take
+// fields on another device, which a kernel would need peer access for.
+inline bool on_this_device(const void* p) {
+  cudaPointerAttributes at;
+  int dev = -1;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == dev);
+}
+
 // Whether work queued on s now goes into a graph that is being captured.
 inline bool stream_captured(cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;

@@ -503,7 +503,7 @@ int to_fourier(sns_ens* e, cudaStream_t s) {
     if (!e->pending[i])
       rc = ns_hist_fourier(e->classes[b.cls].seq, src, dst, 3, s);
     else if (e->turn)
-      rc = op_copy_fields(from, dst, 3, bytes, s);
+      rc = op_copy_fields(from, dst, 3, bytes, nullptr, s);
     if (rc) return rc;
   }
   e->turn = 0;
@@ -865,7 +865,7 @@ int sns_ens_set_state(sns_ens* e, int box, const void* const V1[3], const void* 
   void* const* h = history(e, e->user_to_table[box]);
   const void* src[6] = {V1[0], V1[1], V1[2], cross0[0], cross0[1], cross0[2]};
   void* dst[6] = {b.V[0], b.V[1], b.V[2], h[0], h[1], h[2]};
-  if (int rc = op_copy_fields(src, dst, 6, bytes, e->s)) return rc;
+  if (int rc = op_copy_fields(src, dst, 6, bytes, src, e->s)) return rc;
   if (int rc = mark_fourier(e, e->user_to_table[box])) return rc;
   e->stepped = false;
   return settled(e);
@@ -883,7 +883,8 @@ int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1
   // V1 and its curl from one read of V where both are wanted
   bool both = omega1 && V1 && V1[0] && V1[1] && V1[2];
   for (int i = 0; i < 3 && both; i++)
-    both = omega1[i] && reinterpret_cast<uintptr_t>(V1[i]) % esize_of(e->prec) == 0;
+    both = omega1[i] && reinterpret_cast<uintptr_t>(V1[i]) % esize_of(e->prec) == 0 &&
+           on_this_device(V1[i]);
   if (both) {
     const void* v[3] = {b.V[0], b.V[1], b.V[2]};
     if ((rc = op_curl_copy(v, V1, omega1, d, e->prec, e->s))) return rc;
@@ -904,10 +905,11 @@ int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1
         dst[n++] = cross0[i];
       }
     // a history before its z-forward, or Fourier fields (or a destination that
-    // only a byte copy can write: through the product's fields, free here)
+    // only a copy can write: through the product's fields, free here)
     const bool fourier = e->pending[t] != 0;
     for (int i = 0; i < n && !fourier; i++)
-      if (reinterpret_cast<uintptr_t>(dst[i]) % esize_of(e->prec)) dst[i] = product(e, t)[i];
+      if (reinterpret_cast<uintptr_t>(dst[i]) % esize_of(e->prec) || !on_this_device(dst[i]))
+        dst[i] = product(e, t)[i];
     if (n && !fourier &&
         (rc = ns_hist_fourier(e->classes[b.cls].seq, src, dst, n, e->s)))
       return rc;

@@ -347,14 +347,15 @@ int op_laplacian_inverse(void* f, double a, double b, Dims d, int prec, cudaStre
   return OK;
 }
 
-int op_copy_fields(const void* const* src, void* const* dst, int n, size_t bytes, cudaStream_t s) {
+int op_copy_fields(const void* const* src, void* const* dst, int n, size_t bytes,
+                   const void* const* theirs, cudaStream_t s) {
   // up to 32 MB a field one launch for all (a small copy takes the GPU about as
   // long as a launch: set and read-back of a 32^3 state 19 us of twelve copies);
-  // larger ones, and unaligned ones, a copy each
+  // larger ones, unaligned ones and those of another device a copy each
   bool one = n > 1 && n <= 6 && bytes % 16 == 0 && bytes <= (32u << 20);
   for (int i = 0; i < n && one; i++)
     one = reinterpret_cast<uintptr_t>(src[i]) % 16 == 0 &&
-          reinterpret_cast<uintptr_t>(dst[i]) % 16 == 0;
+          reinterpret_cast<uintptr_t>(dst[i]) % 16 == 0 && (!theirs || on_this_device(theirs[i]));
   if (!one) {
     for (int i = 0; i < n; i++) {
       const int rc = cuda_status(cudaMemcpyAsync(dst[i], src[i], bytes, cudaMemcpyDeviceToDevice, s),

@@ -15,8 +15,10 @@ int op_gradient(const void* f, void* gx, void* gy, void* gz, Dims d, int prec, c
 int op_laplacian(const void* f, void* out, Dims d, int prec, cudaStream_t s);
 int op_laplacian_inverse(void* f, double a, double b, Dims d, int prec, cudaStream_t s);
 // dst[i] = src[i] for n <= 6 fields of `bytes` bytes each, in one launch where the
-// fields are small (any alignment is taken)
-int op_copy_fields(const void* const* src, void* const* dst, int n, size_t bytes, cudaStream_t s);
+// fields are small (any alignment is taken; theirs: src or dst, whichever a caller
+// gave and may lie on any device, null if neither)
+int op_copy_fields(const void* const* src, void* const* dst, int n, size_t bytes,
+                   const void* const* theirs, cudaStream_t s);
 // copy = v and out = i k x v from one read of v
 int op_curl_copy(const void* const v[3], void* const copy[3], void* const out[3], Dims d, int prec,
                  cudaStream_t s);
