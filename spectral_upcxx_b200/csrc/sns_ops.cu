@@ -349,10 +349,11 @@ int op_laplacian_inverse(void* f, double a, double b, Dims d, int prec, cudaStre
 
 int op_copy_fields(const void* const* src, void* const* dst, int n, size_t bytes,
                    const void* const* theirs, cudaStream_t s) {
-  // up to 32 MB a field one launch for all (a small copy takes the GPU about as
-  // long as a launch: set and read-back of a 32^3 state 19 us of twelve copies);
-  // larger ones, unaligned ones and those of another device a copy each
-  bool one = n > 1 && n <= 6 && bytes % 16 == 0 && bytes <= (32u << 20);
+  // up to 2 MB a field one launch for all (a small copy takes the GPU about as
+  // long as a launch).  Six fields set on B200, one launch / six copies, by MB a
+  // field: 0.25 10 / 24 us, 1 10 / 26, 2 15 / 26, 4 27 / 26, 8 49 / 38, 16 62 / 50,
+  // 32 85 / 87.  Larger ones, unaligned ones and those of another device a copy each
+  bool one = n > 1 && n <= 6 && bytes % 16 == 0 && bytes <= (2u << 20);
   for (int i = 0; i < n && one; i++)
     one = reinterpret_cast<uintptr_t>(src[i]) % 16 == 0 &&
           reinterpret_cast<uintptr_t>(dst[i]) % 16 == 0 && (!theirs || on_this_device(theirs[i]));
