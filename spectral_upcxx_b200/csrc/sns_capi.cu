@@ -1018,17 +1018,15 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
     int rc = OK;
     if (cross0 && cross0[0] && cross0[1] && cross0[2]) {
       void* c[3] = {h->C0[0], h->C0[1], h->C0[2]};
-      const bool z = h->hist != HIST_FOURIER;
-      if (z) {
-        for (int i = 0; i < 3; i++) c[i] = nullptr;
-        for (int i = 0; i < 3 && !rc; i++) rc = pool_malloc(&c[i], bytes / 2);
-        if (!rc) rc = ns_hist_fourier(h->pl, h->hist == HIST_Z_U ? h->U : h->C0, c, 3, h->s);
+      if (h->hist != HIST_FOURIER) {
+        // its Fourier form in the fields that the next step builds its product in
+        // (which makes K1's output again, if a step left it there)
+        void* const* from = h->hist == HIST_Z_U ? h->U : h->C0;
+        for (int i = 0; i < 3; i++) c[i] = h->hist == HIST_Z_U ? h->C0[i] : h->U[i];
+        h->carried = false;
+        rc = ns_hist_fourier(h->pl, from, c, 3, h->s);
       }
       if (!rc) rc = convert_half(cross0, c, d.nx, d.ny, d.nz, h->pl.prec, -1, h->s);
-      if (z) {
-        cudaStreamSynchronize(h->s);
-        for (void* p : c) pool_free(p);
-      }
     }
     if (rc || (!omega1 && !(V1 && V1[0] && V1[1] && V1[2]))) return rc;
     void* t[3] = {};
