@@ -755,46 +755,27 @@ struct UpdateArgs {
   int pf_self;
 };
 
-// A divisor shared by several quotients.  FP64: the reciprocal once, each
-// quotient corrected by its remainder (as exact as a division, 3 operations
-// instead of a division's ten or so).  FP32: the reciprocal rounded once.
+// The update's divisors, |k|^2 (a whole number below 2^24) and 1 + nu K/2 |k|^2
+// (formed in FP64).  FP64 quotients are divisions; FP32 ones products with the
+// divisor's reciprocal, rounded once.
 template <typename T>
 struct Divisor {
-  T den, r;
+  T by;
   __device__ __forceinline__ T under(T v) const {
-    if constexpr (sizeof(T) == 8) {
-      const T q = mul_rn(v, r);
-      const T e = fma_rn(-q, den, v);
-      return e == e ? fma_rn(e, r, q) : q;  // an infinite quotient stays infinite
-    } else {
-      return mul_rn(v, r);
-    }
+    if constexpr (sizeof(T) == 8)
+      return v / by;
+    else
+      return mul_rn(v, by);
   }
 };
-// The hardware's FP32 reciprocal (1 ulp).
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-// k2: a whole number below 2^24 (FP32).  The approximate reciprocal improved by
-// one Newton-Raphson step, r (2 - k2 r), whose remainder is exact in an FMA:
-// within 0.500001 ulp, as the FP64 reciprocal rounded to FP32 is.
-__device__ __forceinline__ Divisor<float> divisor_whole(float k2) {
-  const float r = rcp_approx(k2);
-  return {k2, fma_rn(fma_rn(-k2, r, 1.f), r, r)};
-}
-__device__ __forceinline__ Divisor<double> divisor_whole(double k2) { return {k2, 1.0 / k2}; }
-// den >= 1 in FP64.  FP32: one Newton-Raphson step in FP64 from the approximate
-// FP32 reciprocal (relative error about 2^-44 before the rounding to FP32).
+__device__ __forceinline__ Divisor<float> divisor_whole(float k2) { return {__frcp_rn(k2)}; }
+__device__ __forceinline__ Divisor<double> divisor_whole(double k2) { return {k2}; }
 template <typename T>
 __device__ __forceinline__ Divisor<T> divisor_of(double den) {
-  if constexpr (sizeof(T) == 8) {
-    return {den, 1.0 / den};
-  } else {
-    const double r0 = (double)rcp_approx((float)den);
-    return {(T)den, (T)fma_rn(fma_rn(-den, r0, 1.0), r0, r0)};
-  }
+  if constexpr (sizeof(T) == 8)
+    return {den};
+  else
+    return {(T)__drcp_rn(den)};
 }
 
 // Field f of the update's z-forward: the cross product (f < 3) or, with the
