@@ -1169,9 +1169,17 @@ int sns_ns_launches_per_step(sns_ns* h) {
 }
 
 namespace {
-// Tuned plans per device and box: (device, nx, ny, nz, precision, real).
+// Tuned plans per device and box: (device, nx, ny, nz, precision, real) and what
+// the tuner leaves as it is: the pass structure that the environment asked for
+// (xy phase, slabs, K1 carried, K1 as a line pass).
+using TuneKey = std::tuple<int, int, int, int, int, int, int, int>;
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int, int, int>, NSPlan> g_tuned;
+std::map<TuneKey, NSPlan> g_tuned;
+TuneKey tune_key(int dev, const NSPlan& p, bool lines) {
+  const int form = (p.plane ? 1 : 0) | (p.use_xy ? 2 : 0) | (p.use_xyc ? 4 : 0) |
+                   (p.carry ? 8 : 0) | (p.carry_reload ? 16 : 0) | (lines ? 32 : 0);
+  return {dev, p.nx, p.ny, p.nz, p.prec, p.real ? 1 : 0, form, p.xy_chunk};
+}
 }  // namespace
 
 int sns_ns_tune(sns_ns* h) {
@@ -1183,7 +1191,7 @@ int sns_ns_tune(sns_ns* h) {
   int dev = 0;
   cudaGetDevice(&dev);
   const NSPlan& p = h->pl;
-  const auto key = std::make_tuple(dev, p.nx, p.ny, p.nz, p.prec, p.real ? 1 : 0);
+  const auto key = tune_key(dev, p, h->W[0] != nullptr);
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(key);
