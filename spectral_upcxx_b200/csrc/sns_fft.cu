@@ -502,35 +502,46 @@ int fft3d_tune(int nx, int ny, int nz, int nf, int prec, cudaStream_t stream) {
   }
   c.plane = false;
   const int dims[3] = {nx, ny, nz};
-  // the pass of axis a under a candidate plan (its TMA-staged form if chosen)
   int* err_word = fft_tma_err_word();
   auto tma_fits = [&](const FftChoice& q, int a, int S) {
     return S == 0 || (err_word && nf <= 6 &&
                       line_tma_ok(axis_geo(a, nx, ny, nz, prec, q.wmax[a], q.tmax[a], q.ord[a]),
                                   prec, S));
   };
-  auto one = [&](const FftChoice& q, int a, int sg) {
-    const LineGeo g = axis_geo(a, nx, ny, nz, prec, q.wmax[a], q.tmax[a], q.ord[a]);
-    if (q.tma[a] && tma_fits(q, a, q.tma[a]))
-      return run_line_pass_tma(g, f, sg, 0, 1.0, prec, stream, q.tma[a], err_word);
-    return run_line_pass(g, f, sg, 0, 1.0, prec, stream);
+  // the pass of axis a under a candidate plan (its TMA-staged form if chosen; null:
+  // the default plan), as fft3d runs it
+  FftShape shape{};
+  shape.nx = nx;
+  shape.ny = ny;
+  shape.nz = nz;
+  shape.nf = nf;
+  shape.prec = prec;
+  auto one = [&](const FftChoice* q, int a, int sg) {
+    FftShape p = shape;
+    if (q) {
+      p.tuned = true;
+      p.tc = *q;
+      p.err = err_word;
+    }
+    return fft_axis_pass(p, f, a, sg, 0, 1.0, stream);
   };
   for (int a = 0; a < 3 && rc == OK; a++) {
     if (dims[a] < 2) continue;
     // run width (y, z) and thread cap, then radix order, of this axis's pass
     float best = 3.4e38f;
     FftChoice bc = c;
-    for (int W : {4, 8, 16, 32})
-      for (int T : {128, 256, 512})
+    for (int W : {0, 4, 8, 16, 32})  // 0: the default tile
+      for (int T : {0, 64, 128, 256, 512})
         for (int S = 0; S <= 2 && rc == OK; S++) {
-          if (a == 0 && W != 16) continue;  // x lines are single lines
+          if ((W == 0) != (T == 0)) continue;
+          if (a == 0 && W != 0 && W != 16) continue;  // x lines are single lines
           FftChoice q = c;
           q.wmax[a] = W;
           q.tmax[a] = T;
           q.tma[a] = S;
           if (!tma_fits(q, a, S)) continue;
           float t = 0;
-          rc = timed([&](int sg) { return one(q, a, sg); }, &t);
+          rc = timed([&](int sg) { return one(&q, a, sg); }, &t);
           if (rc) break;
           if (getenv("SNS_TUNE_LOG") && getenv("SNS_TUNE_LOG")[0] == '1')
             fprintf(stderr, "fft3d_tune axis=%d W=%d T=%d tma=%d ms=%.4f\n", a, W, T, S, t);
@@ -546,7 +557,7 @@ int fft3d_tune(int nx, int ny, int nz, int nf, int prec, cudaStream_t stream) {
         q.ord[a] = o;
         if (!tma_fits(q, a, q.tma[a])) continue;
         float t = 0;
-        rc = timed([&](int sg) { return one(q, a, sg); }, &t);
+        rc = timed([&](int sg) { return one(&q, a, sg); }, &t);
         if (rc == OK && t < best) {
           best = t;
           bc = q;
@@ -559,8 +570,8 @@ int fft3d_tune(int nx, int ny, int nz, int nf, int prec, cudaStream_t stream) {
   if (rc == OK && fft_xy_supported(nx, ny, nz, nf, prec)) {
     float t_lines = 0, t_plane = 0;
     rc = timed([&](int sg) {
-      int e = one(c, 0, sg);
-      if (!e) e = one(c, 1, sg);
+      int e = one(&c, 0, sg);
+      if (!e) e = one(&c, 1, sg);
       return e;
     }, &t_lines);
     if (rc == OK)
@@ -577,10 +588,7 @@ int fft3d_tune(int nx, int ny, int nz, int nf, int prec, cudaStream_t stream) {
         const int* order = sg < 0 ? axes_fwd : axes_inv;
         const bool plane = ch ? ch->plane : true;
         if (plane && fft_xy_supported(nx, ny, nz, nf, prec)) {
-          auto zpass = [&]() {
-            return ch ? one(*ch, 2, sg)
-                      : run_line_pass(axis_geo(2, nx, ny, nz, prec), f, sg, 0, 1.0, prec, stream);
-          };
+          auto zpass = [&]() { return one(ch, 2, sg); };
           int e = 0;
           if (sg < 0) {
             e = fft_xy_pass(f, nx, nz, sg, 0, 1.0, prec, stream);
@@ -594,9 +602,7 @@ int fft3d_tune(int nx, int ny, int nz, int nf, int prec, cudaStream_t stream) {
         for (int i = 0; i < 3; i++) {
           const int a = order[i];
           if (dims[a] < 2) continue;
-          int e = ch ? one(*ch, a, sg)
-                     : run_line_pass(axis_geo(a, nx, ny, nz, prec), f, sg, 0, 1.0, prec, stream);
-          if (e) return e;
+          if (int e = one(ch, a, sg)) return e;
         }
         return OK;
       }, t);
