@@ -97,11 +97,28 @@ int x_tile_rows(int nx, int64_t rows, int prec) {
   return G;
 }
 
-// Whether the xy phase runs as one CTA per plane: where the plane fits
-// (SNS_PLANE=0: never), unless a form of the separate passes is asked for.
-bool plane_wanted(int nx, int ny, int prec) {
-  if (const char* e = getenv("SNS_PLANE"))
-    if (e[0] == '0') return false;
+// Planes from which one CTA per plane is the faster xy phase.  Planes of up to
+// 16 KB a field: always.  Larger ones take an SM each, for a time that depends on
+// the plane alone, so few of them leave most SMs idle.  Whole steps on B200 in us,
+// five passes / plane: complex64 64 x 64 by planes 16 19.5 / 22.8, 32 24.4 / 25.4,
+// 64 31.0 / 28.4, 256 94 / 82, 1024 711 / 497; 16 x 256 by 4 18.5 / 19.2, 16 22.5 /
+// 20.3; real rows of 256 by 32 64 30.7 / 32.6, 128 47.0 / 40.7; complex128 64 x 32 by
+// 8 19.8 / 22.6, 16 22.9 / 22.3, 32 29.5 / 24.6 (real 16 23.1 / 24.6, 32 30.0 / 26.8).
+// (Beyond, the plane form stays ahead or within 4 %.)
+int plane_least(int nx, int ny, int prec, bool real) {
+  const size_t esz = prec == PREC_C128 ? 16 : 8;
+  if ((size_t)nx * ny * esz <= 16 * 1024) return 0;
+  if (prec == PREC_C128) return real ? 32 : 16;
+  return real ? std::min(2 * nx, 128) : std::min(nx, 64);
+}
+
+// Whether the xy phase runs as one CTA per plane: where the plane fits and there
+// are planes enough (SNS_PLANE=0: never, 1: wherever it fits), unless a form of the
+// separate passes is asked for.
+bool plane_wanted(int nx, int ny, int nz, int prec, bool real) {
+  const char* e = getenv("SNS_PLANE");
+  if (e && e[0] == '0') return false;
+  if (!(e && e[0] == '1') && nz < plane_least(nx, ny, prec, real)) return false;
   for (const char* v : {"SNS_K1_TMA", "SNS_K1_RELOAD", "SNS_K1_SPLIT", "SNS_K1_LINES",
                         "SNS_K1_SMEM_KB", "SNS_X_TMA", "SNS_X_OCC", "SNS_Y_TMA", "SNS_LINE_W",
                         "SNS_RADIX_ORDER", "SNS_Z_TMA", "SNS_Z_W", "SNS_Z_PFSELF", "SNS_CARRY",
@@ -355,7 +372,7 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   }
   pl.k1lW = 0;
   pl.k1lT = 0;
-  pl.plane = !separate && plane_wanted(nx, ny, prec);
+  pl.plane = !separate && plane_wanted(nx, ny, nz, prec, real);
   if (pl.plane) {
     // two launches per step: the plane pass, and the update pass with the next
     // step's K1 carried in it, in CTAs enough for the SMs
