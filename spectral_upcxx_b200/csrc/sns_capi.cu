@@ -605,7 +605,11 @@ int fft1d_lines(void* data, int64_t n, int64_t stride, int64_t howmany, int64_t 
     g.sa = g.W;
   } else {
     g.W = 1;
-    g.G = pow2_divisor(howmany, std::max(1, 256 / TPL));
+    // CTAs of 128 threads: 2^22 elements on B200 in lines of 256 / 512 / 1024, with
+    // 256 threads complex64 16.5 / 20.7 / 23.1 us, complex128 26.9 / 34.0 / 37.3, now
+    // 14.7 / 18.7 / 22.8 and 23.1 / 31.8 / 35.3 (64 threads: the same, but 20.9 against
+    // 17.0 for lines of 4)
+    g.G = pow2_divisor(howmany, std::max(1, 128 / TPL));
     g.gs = dist;
     g.TA = howmany / g.G;
     g.sa = dist * g.G;
