@@ -184,11 +184,18 @@ void* workspace(size_t bytes, cudaStream_t s) {
   return p;
 }
 
-// Populations worth ordering: fields beyond L2, and particles enough that
-// several share what a DRAM access brings.  Not under stream capture (a graph
-// would own the workspace).
+// Populations worth ordering: fields well beyond L2, and particles enough that
+// several share what a DRAM access brings and the two passes over them pay.
+// B200, a move in us as they are / ordered, by MB of the fields: 131 (176^3
+// complex64) 1M 127 / 133, 2.5M 314 / 330; 170 (192^3) 550k 88 / 90, 700k 109 / 105,
+// 1M 152 / 137; 262 (176^3 complex128) 400k 86 / 90, 550k 115 / 106; 403 (256^3) 300k
+// 74 / 83, 550k 127 / 116, 1M 226 / 167; 805 (256^3 complex128) 300k 92 / 102, 550k
+// 153 / 152, 1M 272 / 226; 1359 (384^3) 1M 277 / 249.  Not under stream capture (a
+// graph would own the workspace).
 bool ordered(int64_t np, int64_t n, size_t esz, cudaStream_t s) {
-  if (3.0 * esz * n < 126e6 || np < (1 << 17) || np > 0x7fffffff || np * 64 < n) return false;
+  const double bytes = 3.0 * esz * n;
+  if (bytes < 165e6 || np < (bytes < 250e6 ? 700000 : 550000) || np > 0x7fffffff || np * 64 < n)
+    return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
     cudaGetLastError();
