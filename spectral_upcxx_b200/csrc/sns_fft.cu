@@ -14,6 +14,7 @@
 
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <vector>
 
@@ -530,7 +531,8 @@ int fft3d_tune(int nx, int ny, int nz, int nf, int prec, cudaStream_t stream) {
     // run width (y, z) and thread cap, then radix order, of this axis's pass
     float best = 3.4e38f;
     FftChoice bc = c;
-    for (int W : {0, 4, 8, 16, 32})  // 0: the default tile
+    std::set<std::tuple<int, int, int>> seen;  // tiles timed (thread caps often share one)
+    for (int W : {0, 4, 8, 16, 32})            // 0: the default tile
       for (int T : {0, 64, 128, 256, 512})
         for (int S = 0; S <= 2 && rc == OK; S++) {
           if ((W == 0) != (T == 0)) continue;
@@ -540,6 +542,8 @@ int fft3d_tune(int nx, int ny, int nz, int nf, int prec, cudaStream_t stream) {
           q.tmax[a] = T;
           q.tma[a] = S;
           if (!tma_fits(q, a, S)) continue;
+          const LineGeo g = axis_geo(a, nx, ny, nz, prec, W, T);
+          if (!seen.insert({g.W, g.G, S}).second && T > 64) continue;
           float t = 0;
           rc = timed([&](int sg) { return one(&q, a, sg); }, &t);
           if (rc) break;

@@ -27,6 +27,8 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <set>
+#include <tuple>
 #include <vector>
 
 #include "sns_fft.cuh"
@@ -806,9 +808,12 @@ int ns_tune_plan(NSPlan& pl, void* const V[3], void* const C0[3], void* const U[
   if (rc == OK) {
     c.clear();
     c.push_back(pl);
+    std::set<std::tuple<int, int, int>> seen;  // tiles listed (thread caps often share one)
     for (int W : {4, 8, 16, 32})
       for (int T : {64, 128, 256, 512})
         for (int S = 0; S <= (sync_words ? 2 : 0); S++) {
+          const LineGeo g = axis_geo(1, pl.nx, pl.ny, pl.nz, pl.prec, W, T);
+          if (!seen.insert({g.W, g.G, S}).second) continue;
           NSPlan q = pl;
           q.lineW = W;
           q.lineT = T;
