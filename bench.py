@@ -63,8 +63,7 @@ def pass_names(npasses, plan):
 STEP_FIELDS = 30  # 9 FFTs x 2 + 12 for the spectral update: 30 N^3 S per step
 
 # DRAM bytes (read + write) per launch of each pass at 256^3 complex64 with the
-# tuned plan, from the one-kernel ncu captures summarised in
-# profiles/ns_step_256_c64_launches.md (K1 and K2: their TMA-staged forms).
+# tuned plan, from one-kernel ncu captures (K1 and K2: their TMA-staged forms).
 NCU_TRAFFIC = {
     ("ns256_fp32", "K1 z-inverse+curl"): (404 + 773) * 1e6,
     ("ns256_fp32", "K2 y-inverse x6"): (810 + 749) * 1e6,

@@ -57,8 +57,8 @@ struct EnsClass {
   int nf;         // fields of a line stage
   double scale2;  // 1/N^2 of the cross product
   const void* tw;
-  int pf_self;    // update stage: ask L2 for a tile's V once its cross
-                  // product's loads are in flight
+  int pf_self;    // update stage: ask L2 for a tile's V once its cross product
+                  // and history have been loaded
 };
 
 // Kernel parameter of one stage launch.
@@ -375,9 +375,9 @@ bool make_class(const sns_ens* e, int s, int c, const StageCfg& cfg, EnsClass& k
     k.L = nz;
     k.W = W;
     k.tiles = cols / W;
-    // the update stage's L2 prefetch of V and C0 (SNS_ENS_PFSELF=0: off).
-    // Measured on B200 for 32 x 32^3 + 24 x 64^3 + 8 x 128^3 boxes: update
-    // stage 0.646 against 0.675 ms
+    // the update stage's L2 prefetch of V (SNS_ENS_PFSELF=0: off).  Measured on
+    // B200 for 32 x 32^3 + 24 x 64^3 + 8 x 128^3 boxes: update stage 0.625 against
+    // 0.674 ms (complex128 1.145 against 1.238)
     const char* pe = getenv("SNS_ENS_PFSELF");
     k.pf_self = pe ? (pe[0] == '1') : 1;
     smem = (size_t)3 * W * tile_stride(nz, W, (int)esz) * esz;

@@ -261,7 +261,8 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
     // that fits its stage.  Measured on B200 at 256^3 it does not pay: complex64
     // 0.500 ms (W = 16) and 0.657 (W = 8) against 0.435 direct; complex128
     // 1.159 (W = 8) against 1.016.  The cross product is only a third of the
-    // pass's reads (V and C0 load in the update), the stage and the rows fill
+    // pass's reads (the history joins as its lines load, V in the update), the stage
+    // and the rows fill
     // the SM's shared memory at one CTA, and the persistent tiles add two
     // barriers each.  The tuner still tries it.
     const char* ez = getenv("SNS_Z_TMA");
@@ -288,10 +289,10 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
           pl.zW = w;
           pl.update_blocks = (nx / w) * ny;
         }
-    // L2 prefetch of each tile's V and C0 once its cross product's loads are
-    // in flight (asked before those loads it delayed them), where they come
-    // from HBM (SNS_Z_PFSELF = 0, 1).  B200, 256^3: complex64 0.389 ms against
-    // 0.469 without, complex128 0.776 against 0.894.
+    // L2 prefetch of each tile's V once its cross product and history have been
+    // loaded (asked before those loads it delayed them), where it comes from HBM
+    // (SNS_Z_PFSELF = 0, 1).  B200, 256^3: complex64 0.369 ms against 0.408
+    // without, complex128 0.686 against 0.784.
     const char* epf = getenv("SNS_Z_PFSELF");
     pl.z_pfself = epf ? epf[0] == '1' : big;
     // closure update: nine fields in the tile
@@ -329,8 +330,8 @@ int ns_plan(NSPlan& pl, int nx, int ny, int nz, int prec, int zW, int lineW, boo
   {
     // The y passes of fields beyond L2 over TMA-staged tiles in complex64
     // (SNS_Y_TMA = 0: direct loads, 1 or 2 stages).  B200, 256^3, both passes:
-    // complex64 0.427 ms against 0.491 with direct loads; complex128 0.87
-    // against 0.82.
+    // complex64 0.418 ms against 0.473 with direct loads; complex128 0.85
+    // against 0.75.
     const char* e = getenv("SNS_Y_TMA");
     const int v = e ? atoi(e) : big && prec == PREC_C64 ? 1 : 0;
     pl.y_tma = 0;

@@ -1033,8 +1033,9 @@ __device__ __forceinline__ void zfwd_update_tile(const UpdateArgs& a,
       if (!a.fourier) ab2_rows<E>(a, fld, i0, nxy * TPL, v);
     }
     if (!SGS && a.pf_self) {
-      // with the cross product's loads in flight, ask L2 for this tile's V, so
-      // that the update's loads after the z-forward find it there
+      // the cross product and the history have arrived (a Fourier history: the
+      // former is in flight): ask L2 for this tile's V, so that the update's loads
+      // after the z-forward find it there
 #pragma unroll
       for (int d = 0; d < 3; d++)
         prefetch_lines<L>(reinterpret_cast<const char*>(a.V[d]), base, W, 1, 0, nxy,
