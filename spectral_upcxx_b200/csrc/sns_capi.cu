@@ -324,7 +324,7 @@ struct sns_ns {
   // where the captured calls had them, so from the first such call on every call
   // leaves the history in its Fourier form in C0 (settle, settled).
   bool canonical = false;
-  cudaEvent_t last = nullptr;  // after the steps queued so far
+  cudaEvent_t last = nullptr;  // after the steps and reads queued so far
   // eddy-viscosity closure (none by default) and its six extra work fields
   Closure cl;
   void* U2[6] = {};
@@ -388,7 +388,7 @@ int settle(sns_ns* h, bool* captured) {
   return OK;
 }
 
-// After steps.
+// After a call that read the history or left it somewhere.
 int settled(sns_ns* h) {
   if (h->canonical) return hist_to_fourier(h, h->s);
   if (h->hist == HIST_FOURIER) return OK;
@@ -1011,10 +1011,7 @@ int sns_ns_pass_times(sns_ns* h, double* total_ms, int* launches, int max) {
   return h->pl.passes;
 }
 
-int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* const cross0[3]) {
-  if (!nonnull(h, "sns_ns_get_state")) return ERR_ARG;
-  bool captured;
-  if (int rc = settle(h, &captured)) return rc;
+static int get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* const cross0[3]) {
   if (h->pl.real) {
     // full spectra rebuilt by Hermitian symmetry
     const Dims d{h->pl.nx_phys, h->pl.ny, h->pl.nz};
@@ -1102,6 +1099,15 @@ int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* 
     if ((rc = op_curl(v, omega1, d, h->pl.prec, h->s))) return rc;
   }
   return OK;
+}
+
+int sns_ns_get_state(sns_ns* h, void* const V1[3], void* const omega1[3], void* const cross0[3]) {
+  if (!nonnull(h, "sns_ns_get_state")) return ERR_ARG;
+  bool captured;
+  if (int rc = settle(h, &captured)) return rc;
+  const int rc = get_state(h, V1, omega1, cross0);
+  const int end = settled(h);
+  return rc ? rc : end;
 }
 
 int sns_ns_check(sns_ns* h) {

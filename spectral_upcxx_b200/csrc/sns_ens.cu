@@ -279,7 +279,7 @@ struct sns_ens {
   // every call leaves all histories Fourier in C0, where a replay looks for them
   // (settle, settled)
   bool canonical = false;
-  cudaEvent_t last = nullptr;  // after the steps queued so far
+  cudaEvent_t last = nullptr;  // after the work queued so far
   EnsClass* d_cls = nullptr;  // kEnsStages x nclass
   int64_t* d_parts_ens = nullptr;
   int64_t* d_parts_seq = nullptr;
@@ -871,11 +871,8 @@ int sns_ens_set_state(sns_ens* e, int box, const void* const V1[3], const void* 
   return settled(e);
 }
 
-int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1[3],
-                      void* const cross0[3]) {
-  if (!box_ok(e, box, "sns_ens_get_state")) return ERR_ARG;
-  bool captured;
-  if (int rc = settle(e, &captured)) return rc;
+static int get_state(sns_ens* e, int box, void* const V1[3], void* const omega1[3],
+                     void* const cross0[3]) {
   BoxHost& b = e->boxes[e->user_to_table[box]];
   const Dims d{(int)b.nx, (int)b.ny, (int)b.nz};
   const size_t bytes = esize_of(e->prec) * (size_t)d.n();
@@ -930,6 +927,16 @@ int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1
     if ((rc = op_curl(v, omega1, d, e->prec, e->s))) return rc;
   }
   return OK;
+}
+
+int sns_ens_get_state(sns_ens* e, int box, void* const V1[3], void* const omega1[3],
+                      void* const cross0[3]) {
+  if (!box_ok(e, box, "sns_ens_get_state")) return ERR_ARG;
+  bool captured;
+  if (int rc = settle(e, &captured)) return rc;
+  const int rc = get_state(e, box, V1, omega1, cross0);
+  const int end = settled(e);
+  return rc ? rc : end;
 }
 
 int sns_ens_step(sns_ens* e, int nsteps, int mode) {

@@ -150,3 +150,47 @@ def test_replayed_ensemble_steps_advance_the_state(sns, cuda, mode, n, before):
         del g
         ref.close()
         st.close()
+
+
+@pytest.mark.parametrize("ensemble", [False, True])
+@pytest.mark.parametrize("n", [1, 2])
+def test_reads_still_queued_when_a_capture_begins(sns, cuda, ensemble, n):
+    """A read-back that waits in the stream when the first captured call moves the
+    history to its place for replays reads it where it was."""
+    shape, dtype = (32, 32, 32), torch.complex64
+    a = _state(shape, dtype, cuda, 1)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    N = sns._native
+    with torch.cuda.stream(s):
+        if ensemble:
+            ref, st = (sns.NSEnsemble([shape], [0.01], 1e-4, dtype, tune=False) for _ in range(2))
+            read = lambda q: q.state(0)  # noqa: E731
+        else:
+            ref, st = (sns.NSStepper(shape, 0.01, 1e-4, dtype) for _ in range(2))
+            read = lambda q: q.state()  # noqa: E731
+        for q in (ref, st):
+            q.set_state(0, *a) if ensemble else q.set_state(*a)
+            q.step(2)  # kernels loaded, graphs captured
+            read(q)
+            q.set_state(0, *a) if ensemble else q.set_state(*a)
+            q.step(n)
+        want = read(ref)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(200_000_000)  # about a tenth of a second
+        got = read(st)
+        g = torch.cuda.CUDAGraph()
+        g.capture_begin()
+        st.step(1)
+        g.capture_end()
+        torch.cuda.synchronize()
+        for k in ("V1", "omega1", "cross0"):
+            for x, y in zip(got[k], want[k]):
+                assert torch.equal(x, y), k
+        g.replay()
+        ref.step(1)
+        _close(read(st), read(ref), 1.2e-7)
+        torch.cuda.synchronize()
+        del g
+        ref.close()
+        st.close()
