@@ -6,9 +6,10 @@
 // or 2048 complex128 points each) in shared memory from the y-inverse to the
 // y-forward: one launch, a read of six fields and a write of three instead of
 // 27 field passes.  Steps with it and the carrying update pass against the five
-// passes on B200 (complex64): 32^3 12.0 against 28.7 us, 64^3 30.0 against
-// 35.0 us, 64 x 64 x 256 90 against 104 us; complex128 32^3 16.4 against 32.8
-// us.  At 64 x 64 it is bound by issue on the SMs that hold a plane (45 % of
+// passes on B200 (complex64): 32 x 32 x 64 12.6 against 22.6 us, 64^3 28.4 against
+// 31.0 us, 64 x 64 x 256 82 against 94 us; complex128 32 x 32 x 64 17.7 against 30.2
+// us; few large planes leave SMs idle (the line is at plane_least, sns_ns.cu).  At
+// 64 x 64 it is bound by issue on the SMs that hold a plane (45 % of
 // the slots, one CTA of 24 warps per SM), below by the chain of its five line
 // FFTs.
 #include "../../include/spectral_b200.h"
